@@ -300,3 +300,120 @@ def tolerance(case):
         return "exact"                               # bitmaps, offsets, packed values and codes are defined bit for bit
     # fp16 results, probabilities and dequantised values rounded to fp16, fp32 sums
     return {"rel": 2e-3, "max": 0.05}
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+def _prune(x, rank):
+    size = x.abs().float()
+    return x * (size >= size.kthvalue(rank, dim=-1, keepdim=True).values)
+
+
+def _stored(x, kind, bits, qgroup):
+    """Pruned values as a cache of ``bits``-bit codes stands for them: (code - zero) * scale of each tile's groups."""
+    if bits == 16:
+        return x
+    heads, n, _ = x.shape
+    tiles = (x.view(heads, n // 64, 64, D).transpose(2, 3) if kind == comp.KEY else x.view(heads, n, 2, 64)).float()
+    there, out = tiles != 0, torch.zeros_like(tiles)
+    nth = there.cumsum(-1, dtype=torch.int16) - 1
+    for g in range(64 // qgroup):
+        mine = there & (nth >= g * qgroup) & (nth < (g + 1) * qgroup)
+        lo = tiles.masked_fill(~mine, math.inf).amin(-1, keepdim=True)
+        hi = tiles.masked_fill(~mine, -math.inf).amax(-1, keepdim=True)
+        # tensors divided by tensors: a scalar divisor may be turned into a product with its reciprocal
+        scale = (hi - lo) / torch.full_like(lo, 2 ** bits - 1)
+        scale = torch.where(scale == 0, torch.ones_like(scale), scale)
+        zero = torch.floor(-lo / scale + 0.5).half().float()
+        scale = scale.half().float()
+        code = (torch.floor(tiles / torch.where(scale == 0, torch.ones_like(scale), scale) + 0.5) + zero).clamp(0, 2 ** bits - 1)
+        out = torch.where(mine, (code - zero) * scale, out)
+    return (out.transpose(2, 3) if kind == comp.KEY else out).reshape(heads, n, D)
+
+
+class _Dense:
+    """Takes a store's place in ``_fill`` and keeps the values its cache would stand for."""
+
+    def __init__(self, heads, kind, bits, qgroup):
+        self.n_heads, self.kind, self.bits, self.qgroup, self.parts = heads, kind, bits, qgroup, []
+
+    def append(self, x, rank):
+        step = max(1, (1 << 25) // (x.shape[1] * D))
+        self.parts.append(torch.cat([_stored(_prune(y, rank), self.kind, self.bits, self.qgroup) for y in x.split(step)]))
+
+    def heads(self, lo, hi):
+        return torch.cat([p[lo:hi] for p in self.parts], dim=1).double()
+
+
+def _pair(case, heads):
+    return [_Dense(heads, kind, case.get("bits", 16), case.get("qgroup", 64)) for kind in (comp.KEY, comp.VALUE)]
+
+
+def _attend(k, v, kw, vw, q, group):
+    out, n = [], sum(p.shape[1] for p in k.parts)
+    step = max(1, (1 << 26) // (n * D))
+    for lo in range(0, k.n_heads, step):
+        hi = min(k.n_heads, lo + step)
+        ks, vs = (torch.cat([s.heads(lo, hi), w[lo:hi].double()], 1) for s, w in ((k, kw), (v, vw)))
+        s = q[lo * group:hi * group].double().view(hi - lo, group, D) @ ks.transpose(1, 2) / math.sqrt(D)
+        out.append((s.softmax(-1) @ vs).view(-1, D))
+    return torch.cat(out)
+
+
+def _rmsnorm(x, w):
+    return x * (x.square().mean(-1, keepdim=True) + 1e-5).rsqrt() * w
+
+
+def _rotate(x, angle):
+    a, b = x[..., :D // 2], x[..., D // 2:]
+    return torch.cat([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], -1)
+
+
+def exact(case, seed):
+    what = case["what"]
+    if what not in ("decode", "ops", "step"):
+        return None                                  # nothing but values taken over as they are, and integers
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    rank, g = comp.keep_rank(case["sparsity"]), case["group"]
+    heads, t = case["batch"] * case["kv_heads"], case["tokens"]
+    k, v = _pair(case, heads)
+    if what == "ops":
+        if case["bits"] == 16:
+            _fill(gen, case, k, v, t, _k_scale(gen, heads))
+        else:
+            k.append(_kv(gen, heads, t, _k_scale(gen, heads)), rank)
+            v.append(_kv(gen, heads, t), rank)
+        q = _kv(gen, heads * g, 1)
+        p = torch.softmax(2 * torch.randn(heads * g, 1, t, generator=gen, device=DEV), -1).half()
+        got = [torch.zeros(heads * g, 8, n, dtype=torch.float64, device=DEV) for n in (t, D)]
+        step = max(1, (1 << 26) // (t * D))
+        for lo in range(0, heads, step):
+            hi = min(heads, lo + step)
+            rows = slice(lo * g, hi * g)
+            got[0][rows, 0] = (q[rows].double().view(hi - lo, g, D) @ k.heads(lo, hi).transpose(1, 2)).view(-1, t)
+            got[1][rows, 0] = (p[rows].double().view(hi - lo, g, t) @ v.heads(lo, hi)).view(-1, D)
+        return tuple(got)
+    scale = _k_scale(gen, heads)
+    _fill(gen, case, k, v, t, scale)
+    w = case["window"]
+    if what == "decode":
+        kw, vw = _kv(gen, heads, w, scale), _kv(gen, heads, w)
+        return _attend(k, v, kw, vw, _kv(gen, heads * g, 1)[:, 0], g)
+    b, h, hid, ffn = case["batch"], case["kv_heads"], case["hidden"], case["ffn"]
+    kw, vw = _kv(gen, heads, 384, scale), _kv(gen, heads, 384)
+    rnd = lambda *shape: torch.randn(*shape, generator=gen, device=DEV).half()  # noqa: E731
+    embed, ids = rnd(1000, hid), torch.randint(0, 1000, (b,), generator=gen, device=DEV)
+    qkv, delta, gu = rnd(b, (g + 2) * h * D).double(), rnd(b, hid).double(), rnd(b, 2 * ffn).double()
+    w1, w2 = 1 + 0.1 * rnd(hid), 1 + 0.1 * rnd(hid)
+    angle = (t + w - 1) * 500000.0 ** -(torch.arange(D // 2, dtype=torch.float64, device=DEV) / (D // 2))
+    kw, vw = kw.double(), vw.double()
+    qn, kn, vn = qkv.view(b, (g + 2) * h, D).split([g * h, h, h], dim=1)
+    q = _rotate(qn, angle).reshape(-1, D)
+    kw[:, w - 1], vw[:, w - 1] = _rotate(kn, angle).reshape(-1, D), vn.reshape(-1, D)
+    if case["prune"]:
+        for win in (kw, vw):
+            win[:, w - 130] = _prune(win[:, w - 130], rank)
+    x = embed[ids].double()
+    y = x + delta
+    gate, up = gu.chunk(2, -1)
+    att = _attend(k, v, kw[:, :w], vw[:, :w], q, g)
+    return y, _rmsnorm(x, w1.double()), q, kw, vw, att, _rmsnorm(y, w2.double()), gate * gate.sigmoid() * up
