@@ -7,11 +7,11 @@
 // spmv_kernel: a CTA (4 warps) walks a range of 64-token blocks of ONE kv head and serves all G query heads that
 // share it.  Per block the bitmap array (1 KiB) and the packed-value range travel into a 2-stage shared-memory
 // ring by 1-D bulk copies (cp.async.bulk + mbarrier, no multicast), issued by one thread one block ahead.  Tiles
-// are decoded straight from the bitmap: a lane owns one BYTE of a tile's bitmap (8 positions), 8 lanes cover a
-// tile, a warp does 4 tiles per step; the rank of the lane's first position is the popcount of the bits before its
-// byte; every set bit takes the next packed half and is multiply-accumulated in fp32 for all G heads.
-// KEY: lane owns 8 tokens, loops over its warp's 32 channels.  VALUE: lane owns 8 channels, loops over its warp's
-// 16 tokens; split partials are summed by combine_kernel.
+// become fragments of mma.sync.m16n8k16 the way the fused kernel does it (decode_common.cuh): fp16 products, fp32 sums.
+// KEY: a warp takes 32 channels; the four warps' scores meet in shared memory.  VALUE: a warp takes 16 tokens, whose
+// probabilities it reads from the caller's array as the B operand; split partials are summed by combine_kernel.
+// Against fp32 multiply-adds per position and head: the pair of products over 8 sequences x 16384 tokens with 4 query
+// heads per kv head 177 -> 147 us (the zero fill of the padded scores included).
 #include "decode_common.cuh"
 
 namespace mfar {
@@ -19,59 +19,62 @@ namespace mfar {
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr int kStages = 2;
-// KEY partial planes: (warp, lane group), halved by the shuffle stage that folds two lane groups first
-constexpr int kGroupsPerWarp = 2;
-constexpr int kPlanes = kWarps * kGroupsPerWarp;
+constexpr int kScoreStride = 72;   // floats per (warp, head) score plane: the 32 lanes of a store hit 32 banks
 
 __host__ __device__ inline size_t stage_bytes(int cap) { return 1024 + (static_cast<size_t>(cap) + kSlackHalves) * 2; }
 
-template <int G>
+template <int G, int MODE>
 struct SmemLayout {
-    size_t stages, bars, qs, spart, ps, off, blk, total;
+    size_t stages, bars, red, off, blk, total;
     __host__ __device__ explicit SmemLayout(int cap) {
         size_t o = 0;
+        constexpr size_t sums = static_cast<size_t>(kWarps) * G * kD * 4;
         stages = o; o += kStages * stage_bytes(cap);
+        if (MODE == MODE_VALUE && o < sums) o = sums;
         bars = o;   o += 64;
-        qs = o;     o += kD * G * 2;
-        spart = o;  o += static_cast<size_t>(kPlanes) * G * 64 * 4;   // KEY: score planes; VALUE: [warp][G][128] reduction
-        ps = o;     o += 64 * G * 2;
+        red = MODE == MODE_VALUE ? stages : o;   // VALUE: [warp][G][128] sums, where the ring was; KEY: [warp][G] score planes
+        if (MODE == MODE_KEY) o += static_cast<size_t>(kWarps) * G * kScoreStride * 4;
         off = o;    o += 2 * 128 * 4;
         blk = o;    o += (kMaxBlocksPerSplit + 4) * 4;
         total = o;
     }
 };
-static_assert(kPlanes * 64 >= kWarps * kD, "the VALUE epilogue reuses the score planes as [warp][G][128] floats");
 
 template <int G, int MODE>
-__global__ void __launch_bounds__(kThreads, 4) spmv_kernel(DecodeParams p) {
+__global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
     static_assert(MODE == MODE_KEY || MODE == MODE_VALUE, "single-product kernel");
     extern __shared__ __align__(128) unsigned char smem[];
-    const SmemLayout<G> lay(p.cap);
+    const SmemLayout<G, MODE> lay(p.cap);
     const Sparse& sp = (MODE == MODE_KEY) ? p.k : p.v;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + lay.bars);
-    unsigned short* qs = reinterpret_cast<unsigned short*>(smem + lay.qs);      // [128][G] query, fp16
-    float* spart = reinterpret_cast<float*>(smem + lay.spart);
-    unsigned short* ps = reinterpret_cast<unsigned short*>(smem + lay.ps);      // [64][G] probabilities, fp16
+    float* red = reinterpret_cast<float*>(smem + lay.red);
     unsigned* off = reinterpret_cast<unsigned*>(smem + lay.off);                // [2][128] halves, relative to the block
     int* blk = reinterpret_cast<int*>(smem + lay.blk);                          // block starts (uint32 units) of this split
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // hq numbers the (kv head, set of G query heads) pairs; with kv_share > 1 several of them read the same kv head
-    const int hq = blockIdx.y;
-    const int h = hq / (p.kv_share > 0 ? p.kv_share : 1);
-    const int split = blockIdx.x;
-    const int gi = lane >> 3, kb = lane & 7;
+    const int tb = lane >> 2, cp = lane & 3;   // bitmap byte (fragment row) and tile pair of this lane
+    const int h = blockIdx.y, split = blockIdx.x;
+    const BForms<G> bf(tb, cp);
+    constexpr int FORMS = BForms<G>::FORMS;
     unsigned sel, mh, ml;
-    lane_byte_constants(kb, sel, mh, ml);
+    lane_byte_constants(tb, sel, mh, ml);
 
     const int blk0 = split * p.bps;
     int nb = min(p.bps, p.nblk - blk0);
     if (nb < 0) nb = 0;
 
-    if (MODE == MODE_KEY) {
-        for (int i = tid; i < kD * G; i += kThreads) {
-            const int c = i / G, g = i % G;
-            qs[i] = __half_as_ushort(p.q[(static_cast<int64_t>(hq) * G + g) * p.q_stride + c]);
+    // KEY: query channels warp*32 + 8*g + 2*cp, +1 of head bf.head; VALUE: that head's probabilities
+    unsigned qp[4] = {0u, 0u, 0u, 0u};
+    const __half* prow = nullptr;
+    if (bf.head < G) {
+        const int64_t hq = static_cast<int64_t>(h) * G + bf.head;
+        if (MODE == MODE_KEY) {
+            const __half* qrow = p.q + hq * p.q_stride + warp * 32 + 2 * cp;
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                qp[g] = static_cast<unsigned>(__half_as_ushort(qrow[8 * g])) | (static_cast<unsigned>(__half_as_ushort(qrow[8 * g + 1])) << 16);
+        } else {
+            prow = p.p_in + hq * p.p_stride + static_cast<int64_t>(blk0) * 64 + warp * 16 + 2 * cp;
         }
     }
     const int* acc = sp.acc + h * sp.acc_hs;
@@ -113,11 +116,15 @@ __global__ void __launch_bounds__(kThreads, 4) spmv_kernel(DecodeParams p) {
     }
     __syncthreads();
 
-    float acc_o[8][G];   // VALUE: channels 64*(gi&1) + 8*kb + i, summed over this lane's tokens
+    float dv[2][FORMS][2][4];   // VALUE: channels 64*hf + 8*tb + position of heads bf.ahead, + 1
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
-        for (int g = 0; g < G; ++g) acc_o[i][g] = 0.f;
+        for (int f = 0; f < FORMS; ++f)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dv[hf][f][j][e] = 0.f;
 
     bool timed_out = false;
     for (int i = 0; i < nb; ++i) {
@@ -127,70 +134,70 @@ __global__ void __launch_bounds__(kThreads, 4) spmv_kernel(DecodeParams p) {
         const unsigned* of = off + (i & 1) * 128;
 
         if (i + 1 < nb) fetch_offsets(i + 1);
+        unsigned pp[2] = {0u, 0u};   // VALUE: probabilities of tokens warp*16 + 8*vg + 2*cp, + 1
+        if (MODE == MODE_VALUE && prow) {
+            pp[0] = ldg_nc_u32(prow + static_cast<int64_t>(i) * 64);
+            pp[1] = ldg_nc_u32(prow + static_cast<int64_t>(i) * 64 + 8);
+        }
         if (!mbar_wait(&bars[i % kStages], (i / kStages) & 1)) timed_out = true;
         if (__syncthreads_or(timed_out)) { timed_out = true; break; }   // also publishes the stage hand-off below
         if (tid == 0 && i + kStages - 1 < nb) issue(i + kStages - 1);
 
+        auto expand2 = [&](int tile, unsigned (&r1)[4], unsigned (&r2)[4]) {
+            const uint4 bm = *reinterpret_cast<const uint4*>(bm_s + tile);
+            const uint2 o = *reinterpret_cast<const uint2*>(of + tile);
+            expand_tile(bm.x, bm.y, val + o.x, sel, mh, ml, r1);
+            expand_tile(bm.z, bm.w, val + o.y, sel, mh, ml, r2);
+        };
         if (MODE == MODE_KEY) {
-            float acc_s[8][G];
+            float dk[FORMS][2][4];
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
+            for (int f = 0; f < FORMS; ++f)
 #pragma unroll
-                for (int g = 0; g < G; ++g) acc_s[t][g] = 0.f;
+                for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int s = 0; s < 32 / 4; ++s) {
-                const int c = warp * 32 + s * 4 + gi;
-                const uint2 bm = bm_s[c];
-                unsigned short coef[G];
-                load_coef<G>(qs + c * G, coef);
-                tile_step<G>(bm.y, bm.x, val + of[c], sel, mh, ml, coef, acc_s);
+                    for (int e = 0; e < 4; ++e) dk[f][j][e] = 0.f;
+#pragma unroll
+            for (int kg = 0; kg < 4; ++kg) {
+                unsigned r1[4], r2[4];
+                expand2(warp * 32 + kg * 8 + 2 * cp, r1, r2);
+                mma_step<G>(dk, r1, r2, bf, qp[kg]);
             }
-            // fold two lane groups (same tokens, other channels), the rest meets in partial planes
+            // score planes [warp][head][slot], slot = 8*t + tb for token 8*tb + t
+            float* pl = red + static_cast<size_t>(warp) * G * kScoreStride;
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
+            for (int f = 0; f < FORMS; ++f)
 #pragma unroll
-                for (int g = 0; g < G; ++g) acc_s[t][g] += __shfl_xor_sync(kFull, acc_s[t][g], 16);
-            if (gi < kGroupsPerWarp) {
-                float* dst = spart + (static_cast<size_t>(warp * kGroupsPerWarp + gi) * G) * 64 + kb * 8;
+                for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    *reinterpret_cast<float4*>(dst + g * 64) = make_float4(acc_s[0][g], acc_s[1][g], acc_s[2][g], acc_s[3][g]);
-                    *reinterpret_cast<float4*>(dst + g * 64 + 4) = make_float4(acc_s[4][g], acc_s[5][g], acc_s[6][g], acc_s[7][g]);
-                }
-            }
+                    for (int e = 0; e < 4; ++e) {
+                        const int t = bf.template pos<0>(2 * j + (e >> 1), f);
+                        if (bf.ahead + (e & 1) < G) pl[(bf.ahead + (e & 1)) * kScoreStride + 8 * t + tb] = dk[f][j][e];
+                    }
+            if (i + 1 < nb) store_offsets(i + 1);
             __syncthreads();
+            // lane takes tokens 2*lane, 2*lane + 1 = byte lane / 4, positions 2 * (lane % 4), + 1
             for (int g = warp; g < G; g += kWarps) {
                 float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-                for (int pl = 0; pl < kPlanes; ++pl) {
-                    const float2 t = *reinterpret_cast<const float2*>(spart + (static_cast<size_t>(pl) * G + g) * 64 + 2 * lane);
-                    s0 += t.x;
-                    s1 += t.y;
+                for (int w = 0; w < kWarps; ++w) {
+                    const float* t = red + (static_cast<size_t>(w) * G + g) * kScoreStride + 16 * (lane & 3) + (lane >> 2);
+                    s0 += t[0];
+                    s1 += t[8];
                 }
-                *reinterpret_cast<__half2*>(p.s_out + (static_cast<int64_t>(hq) * G + g) * p.s_stride +
+                *reinterpret_cast<__half2*>(p.s_out + (static_cast<int64_t>(h) * G + g) * p.s_stride +
                                             static_cast<int64_t>(blk0 + i) * 64 + 2 * lane) = __floats2half2_rn(s0, s1);
             }
-            if (i + 1 < nb) store_offsets(i + 1);
         } else {
-            // p comes from the caller: warp j loads heads j, j+4, ...; lane takes tokens 2*lane, 2*lane+1
-            for (int g = warp; g < G; g += kWarps) {
-                const unsigned pv = *reinterpret_cast<const unsigned*>(
-                    p.p_in + (static_cast<int64_t>(hq) * G + g) * p.p_stride + static_cast<int64_t>(blk0 + i) * 64 + 2 * lane);
-                ps[(2 * lane) * G + g] = pv & 0xffffu;
-                ps[(2 * lane + 1) * G + g] = pv >> 16;
-            }
-            if (i + 1 < nb) store_offsets(i + 1);
-            __syncthreads();
-            const int half_id = gi & 1, par = gi >> 1;
 #pragma unroll
-            for (int s = 0; s < 16 / 2; ++s) {
-                const int t = warp * 16 + s * 2 + par;
-                const int tile = half_id * 64 + t;
-                const uint2 bm = bm_s[tile];
-                unsigned short coef[G];
-                load_coef<G>(ps + t * G, coef);
-                tile_step<G>(bm.y, bm.x, val + of[tile], sel, mh, ml, coef, acc_o);
-            }
+            for (int vg = 0; vg < 2; ++vg)
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    unsigned r1[4], r2[4];
+                    expand2(hf * 64 + warp * 16 + vg * 8 + 2 * cp, r1, r2);
+                    mma_step<G>(dv[hf], r1, r2, bf, pp[vg]);
+                }
+            if (i + 1 < nb) store_offsets(i + 1);
         }
     }
 
@@ -200,24 +207,21 @@ __global__ void __launch_bounds__(kThreads, 4) spmv_kernel(DecodeParams p) {
     }
     if (MODE == MODE_KEY) return;
 
-    // ---- VALUE epilogue: join token parities (lanes 16 apart), then the 4 warps, and write the partial
+    // ---- VALUE epilogue: sum the 4 warps and write the partial
     __syncthreads();
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
+    for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
-        for (int g = 0; g < G; ++g) acc_o[t][g] += __shfl_xor_sync(kFull, acc_o[t][g], 16);
-    float* red = spart;   // [warp][G][128]
-    if (lane < 16) {
-        const int ch = (gi & 1) * 64 + kb * 8;
+        for (int f = 0; f < FORMS; ++f)
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float* d = red + (static_cast<size_t>(warp) * G + g) * kD + ch;
-            *reinterpret_cast<float4*>(d) = make_float4(acc_o[0][g], acc_o[1][g], acc_o[2][g], acc_o[3][g]);
-            *reinterpret_cast<float4*>(d + 4) = make_float4(acc_o[4][g], acc_o[5][g], acc_o[6][g], acc_o[7][g]);
-        }
-    }
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int c = hf * 64 + 8 * tb + bf.template pos<0>(2 * j + (e >> 1), f);
+                    if (bf.ahead + (e & 1) < G) red[(static_cast<size_t>(warp) * G + bf.ahead + (e & 1)) * kD + c] = dv[hf][f][j][e];
+                }
     __syncthreads();
-    float* rec = p.ws + ((static_cast<int64_t>(hq) * p.nrec + split) * G) * kPartialStride;
+    float* rec = p.ws + ((static_cast<int64_t>(h) * p.nrec + split) * G) * kPartialStride;
     for (int idx = tid; idx < G * kD; idx += kThreads) {
         const int g = idx / kD, c = idx % kD;
         float s = 0.f;
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(128) combine_kernel(const float* ws, int nrec,
 // ---------------------------------------------------------------------------- host side
 template <int G, int MODE>
 static int launch_spmv(const DecodeParams& p, int n_kv_heads, int grid_x, cudaStream_t s) {
-    const SmemLayout<G> lay(p.cap);
+    const SmemLayout<G, MODE> lay(p.cap);
     static size_t configured[64] = {0};   // largest dynamic shared memory size opted into so far, per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
@@ -304,18 +308,9 @@ static int dispatch_spmv(const DecodeParams& p, int G, int n_kv_heads, int grid_
         case 1: return launch_spmv<1, MODE>(p, n_kv_heads, grid_x, s);
         case 2: return launch_spmv<2, MODE>(p, n_kv_heads, grid_x, s);
         case 4: return launch_spmv<4, MODE>(p, n_kv_heads, grid_x, s);
+        case 8: return launch_spmv<8, MODE>(p, n_kv_heads, grid_x, s);
         default: return MFAR_ERR_ARG;
     }
-}
-
-// 8 query heads per kv head need 64 accumulators per lane and spill; they run as two CTAs of 4 query heads that
-// read the same kv head (the second read hits L2).  Their partial records lie in the
-// [kv head * 2 + half][record][4] layout, which the combine kernel reads with G = 4.
-template <int MODE>
-static int launch_spmv8(const DecodeParams& p, int n_kv_heads, cudaStream_t s) {
-    DecodeParams p2 = p;
-    p2.kv_share = 2;
-    return launch_spmv<4, MODE>(p2, 2 * n_kv_heads, p.nsplit, s);
 }
 
 static int pick_cap(int stage_halves) {
@@ -423,7 +418,6 @@ static int decode_attention_fp16_impl(
     p.nsplit = ns;
     p.bps = ns > 0 ? (p.nblk + ns - 1) / ns : 0;
     p.nrec = ns + (window > 0 ? 1 : 0);
-    p.rec_group = group;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     r = launch_decode_attn(p, group, n_kv_heads, p.nrec, s);
     if (r || p.counters) return r;
@@ -497,7 +491,6 @@ extern "C" int mfar_key_scores_fp16(const void* q, int64_t q_stride, int n_kv_he
     p.s_stride = scores_stride;
     p.dev_status = dev_status;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (group == 8) return launch_spmv8<MODE_KEY>(p, n_kv_heads, s);
     return dispatch_spmv<MODE_KEY>(p, group, n_kv_heads, p.nsplit, s);
 }
 
@@ -531,7 +524,7 @@ extern "C" int mfar_value_output_fp16(const void* probs, int64_t probs_stride, i
     p.ws = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + counters_bytes(n_kv_heads));
     p.dev_status = dev_status;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    r = group == 8 ? launch_spmv8<MODE_VALUE>(p, n_kv_heads, s) : dispatch_spmv<MODE_VALUE>(p, group, n_kv_heads, ns, s);
+    r = dispatch_spmv<MODE_VALUE>(p, group, n_kv_heads, ns, s);
     if (r) return r;
-    return launch_combine(p.ws, ns, group == 8 ? 4 : group, 0, out, out_stride, n_kv_heads * group, s);
+    return launch_combine(p.ws, ns, group, 0, out, out_stride, n_kv_heads * group, s);
 }

@@ -10,22 +10,25 @@
 //
 // Decode: a lane owns one BYTE (8 positions) of the bitmaps of TWO tiles.  The rank of the byte's first position is
 // the popcount of the bitmap bits before it; every set bit then takes the next packed half from shared memory
-// (a predicated 16-bit load), absent positions stay zero, and the two tiles' values at the same position are packed
-// into one 32-bit register.  Those registers ARE fragments of mma.sync.m16n8k16 (fp16 in, fp32 accumulate):
+// (a predicated 16-bit load), absent positions stay zero, and two positions of a tile share a 32-bit register.  Those
+// registers ARE fragments of mma.sync.m16n8k16 (fp16 in, fp32 accumulate):
 //   K phase   S[token][head]   = sum_c K[token][c] q[c][head]     rows = tokens,   k = channels (= K tiles)
 //   V phase   O[channel][head] = sum_t V[t][channel] p[t][head]   rows = channels, k = tokens   (= V tiles)
-// In both phases the position inside a tile is the row and the tile index is the contraction index, which is exactly
-// how the A fragment spreads over a warp (row = lane / 4, k pair = lane % 4), so no transposition is needed.  The
-// query heads (up to 8) are the n dimension.  The multiply-accumulate of a 64-token block is 64 tensor-core
-// instructions per CTA; what remains, and what bounds the kernel, is the shared-memory traffic of the
-// predicated loads.
+// The two positions of a register are told apart by the B operand (BForms in decode_common.cuh): up to 4 query heads
+// fill the 8 columns twice, 8 heads take two instructions.  Against registers that pair two TILES this halves the
+// accumulators of up to 4 heads (128 -> 96 registers, 5 CTAs per SM instead of 4) and the score stores: 64 sequences x
+// 32768 tokens, 4 heads per kv head, 1361 -> 1327 us; 7 x 10176 tokens, 8 heads, 110 -> 106 us.  What bounds the kernel
+// now is the shared-memory traffic of the predicated loads (72 % of the data pipe, 61 % of the issue slots).
 //
 // The same kernel serves the quantised cache (QBITS = 2 or 4): there a tile's code words, bitmap, scale and zero-point
 // are staged by the threads themselves (4-byte cp.async, one tile of each tensor per thread, one block ahead); a lane
-// takes the codes of its byte out of a 32-bit window that starts at its rank, turns every code into
-// fp16((code - zero) * scale) with the subtraction and the product in fp32 - the reference's arithmetic
-// (kernel_quant/csrc/SpMM_Kernel_Quant.cuh:235-240) - and packs the two tiles' values into the same fragments.
-// No per-position shared-memory load is left, so that variant is bound by instruction issue.
+// takes the codes of its byte out of a 32-bit window that starts at its rank, moves them to their positions with two
+// masked shifts (masks from a 2 KiB table indexed by the bitmap byte) and turns them into fp16((code - zero) * scale) two
+// at a time: 2-bit codes by a byte permute out of the tile's four values, which the staging thread computes in fp32 - the
+// reference's arithmetic (kernel_quant/csrc/SpMM_Kernel_Quant.cuh:235-240) -, 4-bit codes by an exact fp16 subtraction
+// and one rounded product, which gives the same bits (zero-points outside +-1024 go through fp32).  Against one
+// predicated step per position: 32 x 16384 tokens of 2-bit codes 583 -> 450 us, 8 x 4096 of 4-bit codes with a scale per
+// 32 nonzeros, half of the values kept, 82.7 -> 69.6 us.  Bound by the integer pipe and issue (both about 60 %).
 #include "decode_common.cuh"
 
 namespace mfar {
@@ -40,8 +43,10 @@ __host__ __device__ inline size_t attn_stage_bytes(int cap) {
     return 2 * (1024 + (static_cast<size_t>(cap) + kSlackHalves) * 2);
 }
 
+struct SpreadTable { uint2 e[256]; };
+
 struct AttnLayout {
-    size_t stages, bars, ps, red, alpha, koff, voff, kblk, vblk, total;
+    size_t stages, bars, ps, red, alpha, koff, voff, kblk, vblk, spread, total;
     size_t s_kbm, s_vbm, s_kval, s_vval;
     // qbuf_bytes > 0: quantised cache, a stage is two QBuf (K then V) instead of bitmaps + packed halves
     __host__ __device__ AttnLayout(int cap, int G, size_t qbuf_bytes = 0) {
@@ -55,42 +60,25 @@ struct AttnLayout {
         ps = o;     o += 8 * kPsStride * 2;
         red = o;    o += static_cast<size_t>(kAWarps) * G * kD * 4;   // score planes, later the output reduction
         alpha = o;  o += 64;
-        koff = o;   o += 2 * 128 * 4;
-        voff = o;   o += 2 * 128 * 4;
-        kblk = o;   o += (kMaxBlocksPerSplit + 4) * 4;
-        vblk = o;   o += (kMaxBlocksPerSplit + 4) * 4;
+        koff = voff = kblk = vblk = spread = o;
+        if (qbuf_bytes) {
+            o += sizeof(SpreadTable);
+        } else {
+            o += 2 * 128 * 4;
+            voff = o;   o += 2 * 128 * 4;
+            kblk = o;   o += (kMaxBlocksPerSplit + 4) * 4;
+            vblk = o;   o += (kMaxBlocksPerSplit + 4) * 4;
+        }
         total = o;
     }
 };
 
-__device__ __forceinline__ void mma16816(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
-                                         unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// byte permute with the full selector (bit 3 of a nibble replicates the byte's sign)
+__device__ __forceinline__ unsigned prmt(unsigned a, unsigned b, unsigned s) {
+    unsigned d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
+    return d;
 }
-
-// Byte `sel` (8 positions) of two tiles -> 8 registers, low half = tile A, high half = tile B, zero where the bit
-// is clear.  bm = {lo A, hi A, lo B, hi B}; va / vb point at the tiles' packed values.
-__device__ __forceinline__ void expand_pair(uint4 bm, const unsigned short* va, const unsigned short* vb, unsigned sel,
-                                            unsigned mh, unsigned ml, unsigned (&r)[8]) {
-    const unsigned ba = __byte_perm(bm.x, bm.y, sel), bb = __byte_perm(bm.z, bm.w, sel);
-    const unsigned short* pa[2];
-    const unsigned short* pb[2];
-    pa[0] = va + (__popc(bm.y & mh) + __popc(bm.x & ml));
-    pb[0] = vb + (__popc(bm.w & mh) + __popc(bm.z & ml));
-    pa[1] = pa[0] + __popc(ba & 0xf0u);
-    pb[1] = pb[0] + __popc(bb & 0xf0u);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        // one zero per register: tile A's half is loaded straight into it, tile B's half is merged in only when present
-        unsigned v = 0;
-        if (ba & (0x80u >> i)) { v = *pa[i / 4]; ++pa[i / 4]; }
-        if (bb & (0x80u >> i)) { const unsigned hi = *pb[i / 4]; ++pb[i / 4]; v = __byte_perm(v, hi, 0x5410); }
-        r[i] = v;
-    }
-}
-
 
 __device__ __forceinline__ void cp_async4(void* dst_smem, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
@@ -98,57 +86,212 @@ __device__ __forceinline__ void cp_async4(void* dst_smem, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// Quantised counterpart of expand_pair: byte `sel` of tiles c and c + 1 of a staged block.  A lane's codes are
-// consecutive in the tile's code words from bit rank * BITS on; every set bit takes the next code.
-template <int BITS, bool GROUP32>
-__device__ __forceinline__ void expand_pair_q(const QBuf<BITS>& b, int c, unsigned sel, unsigned mh, unsigned ml,
-                                              unsigned (&r)[8]) {
-    constexpr unsigned MASK = (1u << BITS) - 1u;
-    constexpr int WPT = QBuf<BITS>::WPT;
-    const uint4 bm = *reinterpret_cast<const uint4*>(&b.bm[c]);
-    const uint4 sz = *reinterpret_cast<const uint4*>(&b.sz[2 * c]);   // (scale | zero << 16): A group 0, 1; B group 0, 1
-    const unsigned ba = __byte_perm(bm.x, bm.y, sel), bb = __byte_perm(bm.z, bm.w, sel);
-    int ra = __popc(bm.y & mh) + __popc(bm.x & ml), rb = __popc(bm.w & mh) + __popc(bm.z & ml);
-    const unsigned oa = static_cast<unsigned>(ra) * BITS, ob = static_cast<unsigned>(rb) * BITS;
-    const unsigned* wa = b.words + c * WPT + (oa >> 5);
-    const unsigned* wb = b.words + (c + 1) * WPT + (ob >> 5);
-    unsigned wina = __funnelshift_r(wa[0], wa[1], oa & 31u), winb = __funnelshift_r(wb[0], wb[1], ob & 31u);
-    auto scale_of = [](unsigned x) { return __half2float(__ushort_as_half(static_cast<unsigned short>(x & 0xffffu))); };
-    // code - zero exactly: the code is or-ed into the mantissa of 2^23, the zero-point is offset by 2^23 as well
-    auto zero_of = [](unsigned x) { return 8388608.f + __half2float(__ushort_as_half(static_cast<unsigned short>(x >> 16))); };
-    const float sa0 = scale_of(sz.x), za0 = zero_of(sz.x), sb0 = scale_of(sz.z), zb0 = zero_of(sz.z);
-    float sa1 = sa0, za1 = za0, sb1 = sb0, zb1 = zb0;
-    if (GROUP32) { sa1 = scale_of(sz.y); za1 = zero_of(sz.y); sb1 = scale_of(sz.w); zb1 = zero_of(sz.w); }
+// ---- quantised tiles
+// A lane's codes are consecutive in the tile's code words from bit rank * BITS on.  They are spread to their positions
+// inside a register, four positions (half a bitmap byte) at a time: an element moves up by the number of absent positions
+// in front of it, first by two (mask `two`, set where such an element arrives), then by one (mask `one`).  Table entry of a
+// bitmap byte (bit 7 = first position), read from shared memory:
+//   2-bit codes: x = two | one << 16 (2 bits per position), y = 4 in the nibble of every absent position
+//   4-bit codes: x = two, y = one (4 bits per position)
+template <int BITS>
+constexpr SpreadTable make_spread_table() {
+    SpreadTable t{};
+    for (unsigned byte = 0; byte < 256; ++byte) {
+        unsigned two = 0, one = 0, absent = 0;
+        for (int half = 0; half < 2; ++half) {
+            int rank = 0;
+            for (int i = 0; i < 4; ++i) {
+                const int pos = 4 * half + i;
+                if ((byte >> (7 - pos)) & 1u) {
+                    const int d = i - rank;
+                    if (d & 2) two |= ((1u << BITS) - 1u) << (BITS * (4 * half + rank + 2));
+                    if (d & 1) one |= ((1u << BITS) - 1u) << (BITS * pos);
+                    ++rank;
+                } else {
+                    absent |= 4u << (4 * pos);
+                }
+            }
+        }
+        t.e[byte].x = BITS == 2 ? (two | one << 16) : two;
+        t.e[byte].y = BITS == 2 ? absent : one;
+    }
+    return t;
+}
+static __device__ const SpreadTable g_spread2 = make_spread_table<2>();
+static __device__ const SpreadTable g_spread4 = make_spread_table<4>();
+
+// One staged tensor of one 64-token block.  par, one entry per 64 or 32 nonzeros of a tile:
+//   2-bit: the four dequantised fp16 values as bytes, x = low bytes, y = high bytes
+//   4-bit: x = scale, y = -(1024 + zero-point), each twice as fp16; a zero-point for which fp16 would not give code - zero
+//          exactly (no integer, or beyond +-1024) has y = kWideZero and x = (scale | zero << 16)
+constexpr unsigned kWideZero = 0xffffffffu;   // a pair of NaNs, which no zero-point in range gives
+template <int BITS_, bool GROUP32>
+struct AttnQBuf {
+    static constexpr int BITS = BITS_;
+    static constexpr int WPT = 64 * BITS_ / 32;  // code words per tile slot
+    static constexpr int NG = GROUP32 ? 2 : 1;
+    uint2 bm[128];
+    uint2 par[128 * NG];
+    unsigned words[128 * WPT + 4];
+};
+
+// (code - zero) * scale in fp32, rounded to fp16 once, for the four 2-bit codes
+__device__ __forceinline__ uint2 dequant_bytes(float scale, float zero) {
+    unsigned v[2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        float va = 0.f, vb = 0.f;
-        if (ba & (0x80u >> i)) {
-            const bool second = GROUP32 && ra >= 32;   // nonzeros 32.. of a tile use the second scale / zero-point
-            va = (__uint_as_float(0x4b000000u | (wina & MASK)) - (second ? za1 : za0)) * (second ? sa1 : sa0);
-            wina >>= BITS;
-            if (GROUP32) ++ra;
-        }
-        if (bb & (0x80u >> i)) {
-            const bool second = GROUP32 && rb >= 32;
-            vb = (__uint_as_float(0x4b000000u | (winb & MASK)) - (second ? zb1 : zb0)) * (second ? sb1 : sb0);
-            winb >>= BITS;
-            if (GROUP32) ++rb;
-        }
-        const __half2 h2 = __floats2half2_rn(va, vb);
-        r[i] = *reinterpret_cast<const unsigned*>(&h2);
+    for (int j = 0; j < 2; ++j) {
+        const __half2 h = __floats2half2_rn((static_cast<float>(2 * j) - zero) * scale, (static_cast<float>(2 * j + 1) - zero) * scale);
+        v[j] = *reinterpret_cast<const unsigned*>(&h);
+    }
+    return make_uint2(__byte_perm(v[0], v[1], 0x6420), __byte_perm(v[0], v[1], 0x7531));
+}
+
+__device__ __forceinline__ uint2 dequant_pair(float scale, float zero, unsigned raw) {
+    if (!(fabsf(zero) <= 1024.f) || zero != rintf(zero)) return make_uint2(raw, kWideZero);
+    const __half2 s = __float2half2_rn(scale), c = __float2half2_rn(-(1024.f + zero));
+    return make_uint2(*reinterpret_cast<const unsigned*>(&s), *reinterpret_cast<const unsigned*>(&c));
+}
+
+// 0xffff per half: bit 7 of byte 0 / bit 7 of byte `second`, replicated (prmt's selectors 8.. copy a byte's sign)
+template <int SECOND>
+__device__ __forceinline__ unsigned half_mask(unsigned x) { return prmt(x, 0u, SECOND == 1 ? 0x9988u : 0xaa88u); }
+
+// 2-bit codes at their positions (4 bits per position, code in the low two) -> pairs (2k, 2k + 1).
+// One value table: 4..7 = absent = the zero operand of the byte permute.
+__device__ __forceinline__ void codes_to_halves2(unsigned codes, uint2 par, unsigned (&r)[4]) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const unsigned c = j ? codes >> 16 : codes;
+        const unsigned l = __byte_perm(par.x, 0u, c), h = __byte_perm(par.y, 0u, c);
+        r[2 * j] = __byte_perm(l, h, 0x5140);
+        r[2 * j + 1] = __byte_perm(l, h, 0x7362);
+    }
+}
+// Two value tables: 4..7 = the second one; absent positions (bit 2 of a nibble of `absent`) are masked.
+__device__ __forceinline__ void codes_to_halves2(unsigned codes, unsigned absent, uint2 par0, uint2 par1, unsigned (&r)[4]) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const unsigned c = j ? codes >> 16 : codes;
+        const unsigned l = __byte_perm(par0.x, par1.x, c), h = __byte_perm(par0.y, par1.y, c);
+        // nibbles of byte j*2 are positions 4j, 4j + 1: bring their bit 2 to bit 7 of two bytes
+        const unsigned a = __byte_perm(absent << 5, absent << 1, j ? 0x7362 : 0x5140);
+        r[2 * j] = __byte_perm(l, h, 0x5140) & ~half_mask<1>(a);
+        r[2 * j + 1] = __byte_perm(l, h, 0x7362) & ~half_mask<1>(a >> 16);
     }
 }
 
-__device__ __forceinline__ unsigned ldg_nc_u32(const void* p) {
-    unsigned v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
+// 4-bit codes at their positions -> pairs (k, k + 4); `present` has one bit per position, first position in bit 7;
+// `later` (two groups) is 0xf at the positions that use the second parameters.
+template <bool GROUP32>
+__device__ __forceinline__ void codes_to_halves4(unsigned codes, unsigned present, unsigned later, uint2 par0, uint2 par1, unsigned (&r)[4]) {
+    const unsigned both = present | (present << 12);   // byte 0: positions 0.., byte 1: positions 4.., first in the top bit
+    if (par0.y == kWideZero || (GROUP32 && par1.y == kWideZero)) {   // rare: the same in fp32
+        float s[2], z[2];
+#pragma unroll
+        for (int g = 0; g < (GROUP32 ? 2 : 1); ++g) {
+            const uint2 par = g ? par1 : par0;
+            const unsigned short sh = static_cast<unsigned short>(par.x & 0xffffu);
+            s[g] = __half2float(__ushort_as_half(sh));
+            z[g] = par.y == kWideZero ? __half2float(__ushort_as_half(static_cast<unsigned short>(par.x >> 16)))
+                                      : -1024.f - __half2float(__ushort_as_half(static_cast<unsigned short>(par.y & 0xffffu)));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int sh = 4 * (k + 4 * e);
+                const bool g = GROUP32 && ((later >> sh) & 1u);
+                v[e] = (static_cast<float>((codes >> sh) & 15u) - (g ? z[GROUP32 ? 1 : 0] : z[0])) * (g ? s[GROUP32 ? 1 : 0] : s[0]);
+            }
+            const __half2 h2 = __floats2half2_rn(v[0], v[1]);
+            r[k] = *reinterpret_cast<const unsigned*>(&h2) & half_mask<1>(both << k);
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        unsigned s = par0.x, c = par0.y;
+        if (GROUP32) {
+            const unsigned m = half_mask<2>(k == 0 ? later << 4 : later >> (4 * (k > 0 ? k - 1 : 0)));
+            s = (s & ~m) | (par1.x & m);
+            c = (c & ~m) | (par1.y & m);
+        }
+        // 1024 + code, minus (1024 + zero): exact, so the one rounding is the product's, as in fp32
+        const unsigned q = ((codes >> (4 * k)) & 0x000f000fu) | 0x64006400u;
+        const __half2 d = __hadd2(*reinterpret_cast<const __half2*>(&q), *reinterpret_cast<const __half2*>(&c));
+        const __half2 v = __hmul2(d, *reinterpret_cast<const __half2*>(&s));
+        r[k] = *reinterpret_cast<const unsigned*>(&v) & half_mask<1>(both << k);
+    }
 }
-__device__ __forceinline__ unsigned ldg_nc_u16(const void* p) {
-    unsigned short v;
-    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
-    return v;
+
+// Codes in packed order (from bit 0) to their positions, both halves of a byte at once: `first` = the nonzeros of its first
+// half.  2-bit codes of one tile in 16 bits; 4-bit codes in 32.
+template <int BITS>
+__device__ __forceinline__ unsigned split_halves(unsigned w, int first) {
+    return __byte_perm(w, w >> (BITS * first), BITS == 2 ? 0x0040 : 0x5410);
 }
+template <int BITS>
+__device__ __forceinline__ unsigned spread_codes(unsigned x, unsigned two, unsigned one) {
+    x = (x & ~two) | ((x << (2 * BITS)) & two);
+    return (x & ~one) | ((x << BITS) & one);
+}
+// 2 -> 4 bits per position: half 0 / 1 of x
+__device__ __forceinline__ unsigned widen_codes(unsigned x, int half) {
+    unsigned y = __byte_perm(x, 0u, half ? 0x4342 : 0x4140);
+    y = (y | (y << 4)) & 0x0f0f0f0fu;
+    return (y | (y << 2)) & 0x33333333u;
+}
+
+// Byte `sel` of tiles c and c + 1 of a staged block.
+template <int BITS, bool GROUP32>
+__device__ __forceinline__ void expand_tiles_q(const AttnQBuf<BITS, GROUP32>& b, const uint2* spread, int c, unsigned sel,
+                                               unsigned mh, unsigned ml, unsigned (&r1)[4], unsigned (&r2)[4]) {
+    constexpr int WPT = AttnQBuf<BITS, GROUP32>::WPT;
+    const uint4 bm = *reinterpret_cast<const uint4*>(&b.bm[c]);
+    unsigned byte[2], win[2], flags[2];
+    uint2 e[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const unsigned lo = t ? bm.z : bm.x, hi = t ? bm.w : bm.y;
+        byte[t] = __byte_perm(lo, hi, sel) & 0xffu;   // the table's index: sel fills the upper bytes with another one
+        e[t] = spread[byte[t]];
+        const unsigned rank = __popc(hi & mh) + __popc(lo & ml);
+        const int first = __popc(byte[t] & 0xf0u);
+        const unsigned o = rank * BITS;
+        const unsigned* w = b.words + (c + t) * WPT + (o >> 5);
+        win[t] = split_halves<BITS>(__funnelshift_r(w[0], w[1], o), first);   // shift taken modulo 32
+        if (GROUP32) {   // all ones for the nonzeros from number 32 of the tile on
+            const int before = max(0, 32 - static_cast<int>(rank));
+            flags[t] = split_halves<BITS>(__funnelshift_lc(0u, 0xffffffffu, BITS * before), first);
+        }
+    }
+    if (BITS == 2) {   // both tiles in one register
+        const unsigned two = __byte_perm(e[0].x, e[1].x, 0x5410), one = __byte_perm(e[0].x, e[1].x, 0x7632);
+        const unsigned x = spread_codes<2>(__byte_perm(win[0], win[1], 0x5410), two, one);
+        if (GROUP32) {
+            const unsigned f = spread_codes<2>(__byte_perm(flags[0], flags[1], 0x5410), two, one);
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+                codes_to_halves2(widen_codes(x, t) | ((widen_codes(f, t) << 1) & 0x44444444u), e[t].y, b.par[(c + t) * 2],
+                                 b.par[(c + t) * 2 + 1], t ? r2 : r1);
+        } else {
+#pragma unroll
+            for (int t = 0; t < 2; ++t) codes_to_halves2(widen_codes(x, t) | e[t].y, b.par[c + t], t ? r2 : r1);
+        }
+    } else {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const unsigned x = spread_codes<4>(win[t], e[t].x, e[t].y);
+            if (GROUP32)
+                codes_to_halves4<true>(x, byte[t], spread_codes<4>(flags[t], e[t].x, e[t].y), b.par[(c + t) * 2], b.par[(c + t) * 2 + 1],
+                                       t ? r2 : r1);
+            else
+                codes_to_halves4<false>(x, byte[t], 0u, b.par[c + t], b.par[c + t], t ? r2 : r1);
+        }
+    }
+}
+
 __device__ __forceinline__ float4 ldcg_f32x4(const float* p) {
     float4 v;
     asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
@@ -162,15 +305,14 @@ __device__ __forceinline__ float ldcg_f32(const float* p) {
 
 // record of (kv head h, split, query head g) inside the workspace
 __device__ __forceinline__ float* record_ptr(const DecodeParams& p, int G, int h, int split, int g) {
-    const int rg = p.rec_group;
-    const int sets = G / rg;
-    return p.ws + ((static_cast<int64_t>(h * sets + g / rg) * p.nrec + split) * rg + (g % rg)) * kPartialStride;
+    return p.ws + ((static_cast<int64_t>(h) * p.nrec + split) * G + g) * kPartialStride;
 }
 
+// 5 CTAs per SM (96 registers); the quantised cache with 8 heads needs two accumulator sets and would spill at 96
 template <int G, int QBITS, bool GROUP32>
-__global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams p) {
+__global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) decode_attn_kernel(DecodeParams p) {
     constexpr bool QUANT = QBITS != 0;
-    using QB = QBuf<QUANT ? QBITS : 2>;
+    using QB = AttnQBuf<QUANT ? QBITS : 2, GROUP32>;
     extern __shared__ __align__(128) unsigned char smem[];
     const AttnLayout lay(p.cap, G, QUANT ? sizeof(QB) : 0);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + lay.bars);
@@ -181,6 +323,7 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
     unsigned* voff = reinterpret_cast<unsigned*>(smem + lay.voff);
     int* kblk = reinterpret_cast<int*>(smem + lay.kblk);                       // block starts (uint32 units) of this split
     int* vblk = reinterpret_cast<int*>(smem + lay.vblk);
+    const uint2* spread = reinterpret_cast<const uint2*>(smem + lay.spread);
     __shared__ int s_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -205,14 +348,21 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
     if (nb < 0) nb = 0;
 
     // ---- prologue
-    // q fragments (B operand of the K phase) of this warp's 32 channels: n = head tb, k pairs 2*cp, 2*cp+1 (+8)
-    unsigned qb[2][2] = {{0u, 0u}, {0u, 0u}};
-    if (tb < G) {
-        const __half* qrow = p.q + (static_cast<int64_t>(h) * G + tb) * p.q_stride + warp * 32 + 2 * cp;
+    const BForms<G> bf(tb, cp);
+    constexpr int FORMS = BForms<G>::FORMS;
+    // query: channels warp*32 + 8*g + 2*cp, +1 of head bf.head (window: head tb, the B operand of its dense layout)
+    unsigned qp[4] = {0u, 0u, 0u, 0u};
+    {
+        const int qh = is_window ? tb : bf.head;
+        if (qh < G) {
+            const __half* qrow = p.q + (static_cast<int64_t>(h) * G + qh) * p.q_stride + warp * 32 + 2 * cp;
 #pragma unroll
-        for (int kg = 0; kg < 2; ++kg)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) qb[kg][j] = ldg_nc_u32(qrow + kg * 16 + j * 8);
+            for (int g = 0; g < 4; ++g) qp[g] = ldg_nc_u32(qrow + 8 * g);
+        }
+    }
+    if (QUANT && !is_window) {
+        const uint2* src = QBITS == 2 ? g_spread2.e : g_spread4.e;
+        for (int i = tid; i < 256; i += kAThreads) const_cast<uint2*>(spread)[i] = src[i];
     }
     for (int i = tid; i < 8 * kPsStride / 2; i += kAThreads) reinterpret_cast<unsigned*>(ps)[i] = 0u;
     const int* kacc = QUANT ? nullptr : p.k.acc + h * p.k.acc_hs;
@@ -281,6 +431,7 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
         m.off = sp.tile_off[mi];
         const int ngrp = GROUP32 ? 2 : 1;
         m.sz[1] = 0u;
+#pragma unroll
         for (int g = 0; g < ngrp; ++g)
             m.sz[g] = static_cast<unsigned>(__half_as_ushort(sp.scales[mi * ngrp + g])) |
                       (static_cast<unsigned>(__half_as_ushort(sp.zeros[mi * ngrp + g])) << 16);
@@ -288,8 +439,13 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
     auto q_stage = [&](const QSparse& sp, const Meta& m, QB& b) {
         constexpr int CAPW = 32 / (QUANT ? QBITS : 2);
         b.bm[tid] = m.bm;
-        b.sz[2 * tid] = m.sz[0];
-        b.sz[2 * tid + 1] = m.sz[1];
+#pragma unroll
+        for (int g = 0; g < QB::NG; ++g) {
+            const float scale = __half2float(__ushort_as_half(static_cast<unsigned short>(m.sz[g] & 0xffffu)));
+            const float zero = __half2float(__ushort_as_half(static_cast<unsigned short>(m.sz[g] >> 16)));
+            b.par[tid * QB::NG + g] = QB::BITS == 2 ? dequant_bytes(scale, zero)
+                                                    : dequant_pair(scale, zero, m.sz[g]);
+        }
         const int n = (__popc(m.bm.x) + __popc(m.bm.y) + CAPW - 1) / CAPW;
         if (m.off < 0 || static_cast<long long>(m.off) + n > sp.packed_words) {
             if (n > 0 && p.dev_status) atomicOr(p.dev_status, MFAR_DEV_BADMETA);
@@ -320,14 +476,17 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
     }
     __syncthreads();
 
-    // running state.  dv[hf][i]: rows = channels 64*hf + 8*tb + i (d0, d1) and + 4 (d2, d3); columns = heads 2*cp, 2*cp+1
-    float dv[2][4][4];
+    // running state.  dv[hf][f][j]: columns = heads bf.ahead, + 1 of form f (G <= 4: bf.aform); rows = the positions of
+    // pair 2*j (d0, d1) and 2*j + 1 (d2, d3) in byte tb, i.e. channels 64*hf + 8*tb + pair_pos
+    float dv[2][FORMS][2][4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int f = 0; f < FORMS; ++f)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) dv[a][i][e] = 0.f;
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dv[a][f][i][e] = 0.f;
     // softmax state of head g lives in warp g % 4: m uniform, l a per-lane partial sum
     constexpr int kHeadsPerWarp = (G + kAWarps - 1) / kAWarps;
     float m_run[kHeadsPerWarp], l_run[kHeadsPerWarp];
@@ -368,39 +527,48 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
         }
 
         // ------------------------------------------------------------ K phase: this warp's 32 channels x 64 tokens
-        // dk[j]: rows = tokens 8*tb + j (d0, d1) and 8*tb + j + 4 (d2, d3); columns = heads 2*cp, 2*cp+1
-        float dk[4][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) dk[j][e] = 0.f;
+        // score planes [warp][head][slot], slot = 8*j + tb for token 8*tb + j (the 32 lanes of a store hit 32 banks)
+        float* pl = red + static_cast<size_t>(warp) * G * kPlaneStride;
         if (!is_window) {
+            float dk[FORMS][2][4];
 #pragma unroll
-            for (int kg = 0; kg < 2; ++kg) {
-                unsigned r1[8], r2[8];
+            for (int f = 0; f < FORMS; ++f)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) dk[f][j][e] = 0.f;
+#pragma unroll
+            for (int kg = 0; kg < 4; ++kg) {
+                unsigned r1[4], r2[4];
+                const int c = warp * 32 + kg * 8 + 2 * cp;
                 if (QUANT) {
-                    const int c = warp * 32 + kg * 16 + 2 * cp;
-                    expand_pair_q<QB::BITS, GROUP32>(qbuf(i, 0), c, sel, mh, ml, r1);
-                    expand_pair_q<QB::BITS, GROUP32>(qbuf(i, 0), c + 8, sel, mh, ml, r2);
+                    expand_tiles_q<QB::BITS, GROUP32>(qbuf(i, 0), spread, c, sel, mh, ml, r1, r2);
                 } else {
-                    {
-                        const int c = warp * 32 + kg * 16 + 2 * cp;
-                        const uint4 bm = *reinterpret_cast<const uint4*>(kbm + c);
-                        const uint2 of = *reinterpret_cast<const uint2*>(ko + c);
-                        expand_pair(bm, kval + of.x, kval + of.y, sel, mh, ml, r1);
-                    }
-                    {
-                        const int c = warp * 32 + kg * 16 + 8 + 2 * cp;
-                        const uint4 bm = *reinterpret_cast<const uint4*>(kbm + c);
-                        const uint2 of = *reinterpret_cast<const uint2*>(ko + c);
-                        expand_pair(bm, kval + of.x, kval + of.y, sel, mh, ml, r2);
-                    }
+                    const uint4 bm = *reinterpret_cast<const uint4*>(kbm + c);
+                    const uint2 of = *reinterpret_cast<const uint2*>(ko + c);
+                    expand_tile(bm.x, bm.y, kval + of.x, sel, mh, ml, r1);
+                    expand_tile(bm.z, bm.w, kval + of.y, sel, mh, ml, r2);
                 }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) mma16816(dk[j], r1[j], r1[j + 4], r2[j], r2[j + 4], qb[kg][0], qb[kg][1]);
+                mma_step<G>(dk, r1, r2, bf, qp[kg]);
             }
+#pragma unroll
+            for (int f = 0; f < FORMS; ++f)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        // token 8*tb + t
+                        const int t = bf.template pos<QBITS>(2 * j + (e >> 1), f);
+                        if (bf.ahead + (e & 1) < G) pl[(bf.ahead + (e & 1)) * kPlaneStride + 8 * t + tb] = dk[f][j][e];
+                    }
         } else {
-            // dense window: the A fragment is two adjacent channels of one token, a 32-bit load
+            // dense window: the A fragment is two adjacent channels of one token, a 32-bit load; rows = tokens 8*tb + j
+            // (d0, d1) and + 4 (d2, d3), columns = heads 2*cp, 2*cp + 1
+            float dk[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dk[j][e] = 0.f;
             const __half* kw = p.kwin + h * p.win_hs;
 #pragma unroll
             for (int kg = 0; kg < 2; ++kg) {
@@ -411,27 +579,14 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
                     unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0;
                     if (t0 < W) { a0 = ldg_nc_u32(kw + t0 * p.win_ts + c); a2 = ldg_nc_u32(kw + t0 * p.win_ts + c + 8); }
                     if (t1 < W) { a1 = ldg_nc_u32(kw + t1 * p.win_ts + c); a3 = ldg_nc_u32(kw + t1 * p.win_ts + c + 8); }
-                    mma16816(dk[j], a0, a1, a2, a3, qb[kg][0], qb[kg][1]);
+                    mma16816(dk[j], a0, a1, a2, a3, qp[2 * kg], qp[2 * kg + 1]);
                 }
             }
-        }
-        // score planes [warp][head][slot], slot = 8*j + tb for token 8*tb + j (consecutive lanes, consecutive words)
-        {
-            float* pl = red + static_cast<size_t>(warp) * G * kPlaneStride;
-            if (2 * cp < G) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    pl[(2 * cp) * kPlaneStride + j * 8 + tb] = dk[j][0];
-                    pl[(2 * cp) * kPlaneStride + (j + 4) * 8 + tb] = dk[j][2];
-                }
-            }
-            if (2 * cp + 1 < G) {
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    pl[(2 * cp + 1) * kPlaneStride + j * 8 + tb] = dk[j][1];
-                    pl[(2 * cp + 1) * kPlaneStride + (j + 4) * 8 + tb] = dk[j][3];
-                }
-            }
+                for (int e = 0; e < 4; ++e)
+                    if (2 * cp + (e & 1) < G) pl[(2 * cp + (e & 1)) * kPlaneStride + (j + 4 * (e >> 1)) * 8 + tb] = dk[j][e];
         }
         __syncthreads();
 
@@ -473,63 +628,54 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
         // ------------------------------------------------------------ V phase: this warp's 16 tokens x 128 channels
         {
             float a0 = 1.f, a1 = 1.f;
-            if (2 * cp < G) a0 = alpha_s[2 * cp];
-            if (2 * cp + 1 < G) a1 = alpha_s[2 * cp + 1];
+            if (bf.ahead < G) a0 = alpha_s[bf.ahead];
+            if (bf.ahead + 1 < G) a1 = alpha_s[bf.ahead + 1];
             if (__any_sync(kFull, a0 != 1.f || a1 != 1.f)) {
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf)
+                for (int f = 0; f < FORMS; ++f)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        dv[hf][j][0] *= a0; dv[hf][j][1] *= a1;
-                        dv[hf][j][2] *= a0; dv[hf][j][3] *= a1;
-                    }
+                    for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            dv[hf][f][j][0] *= a0; dv[hf][f][j][1] *= a1;
+                            dv[hf][f][j][2] *= a0; dv[hf][f][j][3] *= a1;
+                        }
             }
         }
-        // probabilities as the B operand: n = head tb, k pairs = tokens 16*warp + 2*cp, +1 (+8)
-        const unsigned pb0 = *reinterpret_cast<const unsigned*>(ps + tb * kPsStride + warp * 16 + 2 * cp);
-        const unsigned pb1 = *reinterpret_cast<const unsigned*>(ps + tb * kPsStride + warp * 16 + 8 + 2 * cp);
-        if (!is_window) {
+        // a tile is 64 channels of one token; the window's values have the same shape, read as 32-bit pairs of channels
+#pragma unroll
+        for (int vg = 0; vg < 2; ++vg) {
+            const int t = warp * 16 + vg * 8 + 2 * cp;
+            const unsigned pp = *reinterpret_cast<const unsigned*>(ps + bf.head * kPsStride + t);   // tokens t, t + 1
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                unsigned r1[8], r2[8];
-                if (QUANT) {
-                    const int t = hf * 64 + warp * 16 + 2 * cp;
-                    expand_pair_q<QB::BITS, GROUP32>(qbuf(i, 1), t, sel, mh, ml, r1);
-                    expand_pair_q<QB::BITS, GROUP32>(qbuf(i, 1), t + 8, sel, mh, ml, r2);
+                unsigned r1[4], r2[4];
+                if (!is_window) {
+                    if (QUANT) {
+                        expand_tiles_q<QB::BITS, GROUP32>(qbuf(i, 1), spread, hf * 64 + t, sel, mh, ml, r1, r2);
+                    } else {
+                        const uint4 bm = *reinterpret_cast<const uint4*>(vbm + hf * 64 + t);
+                        const uint2 of = *reinterpret_cast<const uint2*>(vo + hf * 64 + t);
+                        expand_tile(bm.x, bm.y, vval + of.x, sel, mh, ml, r1);
+                        expand_tile(bm.z, bm.w, vval + of.y, sel, mh, ml, r2);
+                    }
                 } else {
-                    {
-                        const int t = hf * 64 + warp * 16 + 2 * cp;
-                        const uint4 bm = *reinterpret_cast<const uint4*>(vbm + t);
-                        const uint2 of = *reinterpret_cast<const uint2*>(vo + t);
-                        expand_pair(bm, vval + of.x, vval + of.y, sel, mh, ml, r1);
-                    }
-                    {
-                        const int t = hf * 64 + warp * 16 + 8 + 2 * cp;
-                        const uint4 bm = *reinterpret_cast<const uint4*>(vbm + t);
-                        const uint2 of = *reinterpret_cast<const uint2*>(vo + t);
-                        expand_pair(bm, vval + of.x, vval + of.y, sel, mh, ml, r2);
-                    }
+                    const __half* vw = p.vwin + h * p.win_hs + hf * 64 + 8 * tb;
+                    auto row = [&](int tok, unsigned (&r)[4]) {
+                        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                        if (tok < W) x = ldg_nc_u4(vw + tok * p.win_ts);
+                        if (pair_pos<QBITS>(0, 1) == 1) {
+                            r[0] = x.x; r[1] = x.y; r[2] = x.z; r[3] = x.w;
+                        } else {
+                            r[0] = __byte_perm(x.x, x.z, 0x5410); r[1] = __byte_perm(x.x, x.z, 0x7632);
+                            r[2] = __byte_perm(x.y, x.w, 0x5410); r[3] = __byte_perm(x.y, x.w, 0x7632);
+                        }
+                    };
+                    row(i * 64 + t, r1);
+                    row(i * 64 + t + 1, r2);
                 }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) mma16816(dv[hf][j], r1[j], r1[j + 4], r2[j], r2[j + 4], pb0, pb1);
+                mma_step<G>(dv[hf], r1, r2, bf, pp);
             }
-        } else {
-            // dense window: the A fragment pairs two adjacent tokens of one channel (two 16-bit loads)
-            const __half* vw = p.vwin + h * p.win_hs;
-            const int tA = i * 64 + warp * 16 + 2 * cp;
-            auto pair = [&](int t, int ch) -> unsigned {
-                unsigned lo = 0, hi = 0;
-                if (t < W) lo = ldg_nc_u16(vw + t * p.win_ts + ch);
-                if (t + 1 < W) hi = ldg_nc_u16(vw + (t + 1) * p.win_ts + ch);
-                return __byte_perm(lo, hi, 0x5410);
-            };
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c0 = hf * 64 + 8 * tb + j, c1 = c0 + 4;
-                    mma16816(dv[hf][j], pair(tA, c0), pair(tA, c1), pair(tA + 8, c0), pair(tA + 8, c1), pb0, pb1);
-                }
         }
     }
 
@@ -539,19 +685,17 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
     // that the merge below still sees every record arrive)
     __syncthreads();
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf)
+    for (int f = 0; f < FORMS; ++f)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c0 = hf * 64 + 8 * tb + j, c1 = c0 + 4;
-            if (2 * cp < G) {
-                red[(static_cast<size_t>(warp) * G + 2 * cp) * kD + c0] = dv[hf][j][0];
-                red[(static_cast<size_t>(warp) * G + 2 * cp) * kD + c1] = dv[hf][j][2];
-            }
-            if (2 * cp + 1 < G) {
-                red[(static_cast<size_t>(warp) * G + 2 * cp + 1) * kD + c0] = dv[hf][j][1];
-                red[(static_cast<size_t>(warp) * G + 2 * cp + 1) * kD + c1] = dv[hf][j][3];
-            }
-        }
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int c = bf.template pos<QBITS>(2 * j + (e >> 1), f);
+                    const int g = bf.ahead + (e & 1);
+                    if (g < G) red[(static_cast<size_t>(warp) * G + g) * kD + hf * 64 + 8 * tb + c] = dv[hf][f][j][e];
+                }
     __syncthreads();
     for (int idx = tid; idx < G * kD; idx += kAThreads) {
         const int g = idx / kD, c = idx % kD;
@@ -592,7 +736,7 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
     float* wgt = red;   // [G][nrec], nrec <= 129
     for (int g = warp; g < G; g += kAWarps) {
         const float* base = record_ptr(p, G, h, 0, g);
-        const int64_t step = static_cast<int64_t>(p.rec_group) * kPartialStride;
+        const int64_t step = static_cast<int64_t>(G) * kPartialStride;
         float M = -INFINITY;
         for (int s = lane; s < nrec; s += 32) M = fmaxf(M, ldcg_f32(base + s * step + kPartM));
         M = warp_max_f32(M);
@@ -634,7 +778,7 @@ __global__ void __launch_bounds__(kAThreads, 4) decode_attn_kernel(DecodeParams 
 
 template <int G, int QBITS, bool GROUP32>
 static int launch_attn(const DecodeParams& p, int n_kv_heads, int grid_x, cudaStream_t s) {
-    const AttnLayout lay(p.cap, G, QBITS ? sizeof(QBuf<QBITS ? QBITS : 2>) : 0);
+    const AttnLayout lay(p.cap, G, QBITS ? sizeof(AttnQBuf<QBITS ? QBITS : 2, GROUP32>) : 0);
     static size_t configured[64] = {0};   // largest dynamic shared memory size opted into so far, per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;

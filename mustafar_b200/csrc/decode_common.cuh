@@ -1,6 +1,6 @@
 // Building blocks shared by the fp16 and the quantised decode kernels:
-// mbarrier / bulk-copy wrappers (1-D cp.async.bulk, no multicast), the position-centric
-// tile step, the split-KV partial record and the launch parameters.
+// mbarrier / bulk-copy wrappers (1-D cp.async.bulk, no multicast), the expansion of bitmap tiles
+// into tensor-core fragments, the split-KV partial record and the launch parameters.
 #pragma once
 
 #include "common.cuh"
@@ -65,43 +65,85 @@ __device__ __forceinline__ float warp_sum_f32(float v) {
     return v;
 }
 
-// One tile step for one lane.  `hi:lo` is the tile's 64-bit bitmap (bit 63-i = element i),
-// `vals` its packed values in shared memory.  The lane owns byte `kb` of the bitmap, i.e.
-// positions 8*kb .. 8*kb+7: sel / mh / ml are the lane constants that extract that byte and
-// mask the bits in front of it.  The rank of the lane's first position is the popcount of
-// the bits before its byte; every set bit then consumes the next packed half and is
-// multiply-accumulated in fp32 into acc[i][g] with the per-tile coefficients coef[g]
-// (K phase: the query channel; V phase: the probability of the token).  The compiler turns
-// the `if` into predicated instructions (no branch, no zero fill).
+// A lane owns byte `kb` of a tile's 64-bit bitmap (bit 63-i = element i), i.e. positions 8*kb .. 8*kb+7: sel / mh / ml
+// are the lane constants that extract that byte and mask the bits in front of it (hi, lo = the bitmap's words).  The rank
+// of the lane's first position is the popcount of the bits before its byte.
 __device__ __forceinline__ void lane_byte_constants(int kb, unsigned& sel, unsigned& mh, unsigned& ml) {
     sel = 7u - kb;
     mh = kb == 0 ? 0u : (kb >= 4 ? 0xffffffffu : (0xffffffffu << (32 - 8 * kb)));
     ml = kb <= 4 ? 0u : (0xffffffffu << (64 - 8 * kb));
 }
 
-__device__ __forceinline__ float fma_h(float acc, unsigned short a, unsigned short b) {
-    asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(acc) : "h"(a), "h"(b));
-    return acc;
+__device__ __forceinline__ unsigned ldg_nc_u32(const void* p) {
+    unsigned v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
 
-// The packed half and the fp16 coefficient go straight into one mixed-precision FMA (fp16 x fp16 + fp32, full rate
-// on sm_100).  Two read pointers (positions 0-3 and 4-7) keep the dependent chain of pointer bumps short.
-template <int G>
-__device__ __forceinline__ void tile_step(unsigned hi, unsigned lo, const unsigned short* vals, unsigned sel,
-                                          unsigned mh, unsigned ml, const unsigned short (&coef)[G], float (&acc)[8][G]) {
+// ---------------------------------------------------------------- tensor-core fragments of decoded tiles
+__device__ __forceinline__ void mma16816(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
+                                         unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// A fragments: register k of a tile's byte holds two of its 8 positions, pair_pos(k, 0) in the low half and
+// pair_pos(k, 1) in the high half, zero where the bit is clear.  Which two is free (the B operand tells them apart):
+// fp16 values and 4-bit codes pair k with k + 4, 2-bit codes 2k with 2k + 1.
+template <int QBITS>
+__host__ __device__ constexpr int pair_pos(int k, int par) { return QBITS == 2 ? 2 * k + par : k + 4 * par; }
+
+// One tile of packed halves: every set bit of byte `sel` takes the next half (a predicated load); the two half bytes
+// have a read pointer each.
+__device__ __forceinline__ void expand_tile(unsigned lo, unsigned hi, const unsigned short* vals, unsigned sel, unsigned mh,
+                                            unsigned ml, unsigned (&r)[4]) {
     const unsigned byte = __byte_perm(lo, hi, sel);
-    const unsigned short* pv[2];
-    pv[0] = vals + (__popc(hi & mh) + __popc(lo & ml));
-    pv[1] = pv[0] + __popc(byte & 0xf0u);
+    const unsigned short* p0 = vals + (__popc(hi & mh) + __popc(lo & ml));
+    const unsigned short* p1 = p0 + __popc(byte & 0xf0u);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if (byte & (0x80u >> i)) {
-            const unsigned short*& p = pv[i / 4];
-            const unsigned short v = *p;
-            ++p;
+    for (int k = 0; k < 4; ++k) {
+        unsigned v = 0;
+        if (byte & (0x80u >> k)) { v = *p0; ++p0; }
+        if (byte & (0x08u >> k)) { const unsigned h = *p1; ++p1; v = __byte_perm(v, h, 0x5410); }
+        r[k] = v;
+    }
+}
+
+// Where a tile's coefficient (query channel, probability) goes in the B operand: a register of A holds two positions of
+// ONE tile, so it enters B as (c, 0) for the first position and as (0, c) for the second.  Up to 4 query heads fill the 8
+// columns with both forms (column = head + 4 * form); 8 heads take one mma per form.
+template <int G>
+struct BForms {
+    static constexpr int FORMS = G == 8 ? 2 : 1;
+    int head;              // query head whose coefficients this lane loads
+    unsigned sel0, sel1;   // place the low / high half of a register of two adjacent tiles' coefficients
+    int ahead, aform;      // head of accumulator column 2*cp (and + 1), and its form (G <= 4)
+    __device__ __forceinline__ BForms(int tb, int cp) {
+        head = G == 8 ? tb : (tb & 3);
+        const bool second = G != 8 && tb >= 4;
+        sel0 = second ? 0x1044u : 0x4410u;
+        sel1 = second ? 0x3244u : 0x4432u;
+        ahead = G == 8 ? 2 * cp : 2 * (cp & 1);
+        aform = G == 8 ? 0 : cp >> 1;
+    }
+    // position inside the lane's byte of register k of an accumulator of form f
+    template <int QBITS>
+    __device__ __forceinline__ int pos(int k, int f) const {
+        return FORMS == 2 ? pair_pos<QBITS>(k, f) : (aform ? pair_pos<QBITS>(k, 1) : pair_pos<QBITS>(k, 0));
+    }
+};
+
+// d[f][j] += the eight tiles of a step (r1: tile 2*cp, r2: tile 2*cp + 1 of the lane's column) times their coefficients cc
+template <int G>
+__device__ __forceinline__ void mma_step(float (&d)[BForms<G>::FORMS][2][4], const unsigned (&r1)[4], const unsigned (&r2)[4],
+                                         const BForms<G>& bf, unsigned cc) {
+    const unsigned b0 = __byte_perm(cc, 0u, bf.sel0), b1 = __byte_perm(cc, 0u, bf.sel1);
 #pragma unroll
-            for (int g = 0; g < G; ++g) acc[i][g] = fma_h(acc[i][g], v, coef[g]);
-        }
+    for (int j = 0; j < 2; ++j) {
+        mma16816(d[0][j], r1[2 * j], r1[2 * j + 1], r2[2 * j], r2[2 * j + 1], b0, b1);
+        if (BForms<G>::FORMS == 2)
+            mma16816(d[BForms<G>::FORMS - 1][j], r1[2 * j], r1[2 * j + 1], r2[2 * j], r2[2 * j + 1], b0 << 16, b1 << 16);
     }
 }
 
@@ -120,32 +162,6 @@ __device__ __forceinline__ void load_coef(const float* p, float (&c)[G]) {
         }
     }
 }
-
-template <int G>
-__device__ __forceinline__ void load_coef(const unsigned short* p, unsigned short (&c)[G]) {
-    if constexpr (G == 1) {
-        c[0] = p[0];
-    } else if constexpr (G == 2) {
-        const unsigned t = *reinterpret_cast<const unsigned*>(p);
-        c[0] = t & 0xffffu; c[1] = t >> 16;
-    } else {
-#pragma unroll
-        for (int g = 0; g < G; g += 4) {
-            const uint2 t = *reinterpret_cast<const uint2*>(p + g);
-            c[g] = t.x & 0xffffu; c[g + 1] = t.x >> 16; c[g + 2] = t.y & 0xffffu; c[g + 3] = t.y >> 16;
-        }
-    }
-}
-
-__device__ __forceinline__ void store_coef(float* p, float v) { *p = v; }
-__device__ __forceinline__ void store_coef(unsigned short* p, float v) { *p = __half_as_ushort(__float2half_rn(v)); }
-__device__ __forceinline__ float coef_value(float v) { return v; }
-// the probability that enters P.V is the fp16-rounded one; the running sum must use the same value
-__device__ __forceinline__ float round_like(const unsigned short*, float v) { return __half2float(__float2half_rn(v)); }
-__device__ __forceinline__ float round_like(const float*, float v) { return v; }
-
-__device__ __forceinline__ float coef_to_float(float v) { return v; }
-__device__ __forceinline__ float coef_to_float(unsigned short v) { return __half2float(__ushort_as_half(v)); }
 
 // Split-KV partial of one (kv head, split, q head of the group): 128 un-normalised
 // output channels, then the running max (log2 domain) and the running sum.
@@ -202,14 +218,12 @@ struct DecodeParams {
     float scale_log2;      // softmax scale * log2(e)
     float* ws;             // split partials
     int nrec;              // partial records per kv head in ws
-    int rec_group;         // query heads per record set: G, or 4 when 8 heads are laid out as two sets of 4
     __half* s_out;         // MODE_KEY  : [Bq][s_stride]
     int64_t s_stride;
     const __half* p_in;    // MODE_VALUE: [Bq][p_stride]
     int64_t p_stride;
     unsigned* dev_status;
     int split_offset;      // added to blockIdx.x (lets a launch cover only the window record)
-    int kv_share;          // single-product kernels: grid rows (sets of query heads) sharing one kv head; 0 reads as 1
     // fused attention only: the CTA that finishes a kv head last merges its records into out
     unsigned* counters;    // one per kv head, zero between launches; NULL = no merge (a combine launch follows)
     __half* out;

@@ -468,7 +468,6 @@ extern "C" int mfar_decode_attention_quant(
     p.out = static_cast<__half*>(out);
     p.out_stride = out_stride;
     p.dev_status = dev_status;
-    p.rec_group = group;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     r = launch_decode_attn_quant(p, group, bits, qgroup == 32, n_kv_heads, p.nrec, s);
     if (r || p.counters) return r;
