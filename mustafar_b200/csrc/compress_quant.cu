@@ -22,7 +22,7 @@ struct QuantParams {
     int64_t xhs, xts;
     int hpg;                       // heads per group (0: one stride for all heads)
     int64_t xgs;                   // stride between groups of heads
-    int n_heads, nblk, rank, bits, group;
+    int n_heads, nblk, rank;
     unsigned long long* bmp;
     int* tile_off;
     int* counts;
@@ -60,8 +60,21 @@ __device__ __forceinline__ GroupQ make_group(float xmin, float xmax, bool has, i
     return g;
 }
 
-template <int KIND>
+// smallest and largest kept value of a tile, as fp16 (a kept value is never zero, so the order of +0 and -0 is moot)
+struct TileRange {
+    __half lo, hi;
+    __device__ __forceinline__ TileRange() : lo(__ushort_as_half(0x7c00)), hi(__ushort_as_half(0xfc00)) {}
+    __device__ __forceinline__ void add(unsigned short v) {
+        lo = __hmin(lo, __ushort_as_half(v));
+        hi = __hmax(hi, __ushort_as_half(v));
+    }
+};
+
+template <int KIND, int BITS, int GROUP>
 __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
+    constexpr int maxq = (1 << BITS) - 1;
+    constexpr int cap = 32 / BITS;             // codes per word
+    constexpr int ngrp = 64 / GROUP;
     __shared__ __align__(16) unsigned short vals[64 * 128];                                     // kept values, tile order, no padding
     __shared__ __align__(16) unsigned short xs[KIND == MFAR_KIND_KEY ? 64 * kXsStride : 8];     // K: the raw block
     __shared__ unsigned s_mask[4][64];       // K: keep flags [32-channel word][row], first channel in the top bit
@@ -81,9 +94,6 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
     const int h = static_cast<int>(s_ticket) / p.nblk;
     const int b = static_cast<int>(s_ticket) % p.nblk;
     if (h >= p.n_heads) return;
-    const int maxq = (1 << p.bits) - 1;
-    const int cap = 32 / p.bits;
-    const int ngrp = 64 / p.group;
 
     // ---- the pair loads one row, selects the threshold, ends up with one "kept and nonzero" flag per element
     uint4 v[8];
@@ -172,16 +182,26 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
     const int chain_first = compact ? 0 : h * p.nblk;
     if (tid == 0) lookback_announce(p.state, pos, chain_first, total);
 
-    // ---- kept values into vals, tile order (K: down the columns of the raw block; V: from the registers)
+    // ---- kept values into vals, tile order (K: down the columns of the raw block; V: from the registers).  With one
+    // parameter group per tile its range is taken on the way; with two, the rank of a value decides its group (below)
+    TileRange range;
     if (KIND == MFAR_KIND_KEY) {
         unsigned o = voff;
         const int c = tid;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-            if ((hi >> (31 - i)) & 1u) vals[o++] = xs[i * kXsStride + c];
+            if ((hi >> (31 - i)) & 1u) {
+                const unsigned short v = xs[i * kXsStride + c];
+                vals[o++] = v;
+                if (ngrp == 1) range.add(v);
+            }
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-            if ((lo >> (31 - i)) & 1u) vals[o++] = xs[(32 + i) * kXsStride + c];
+            if ((lo >> (31 - i)) & 1u) {
+                const unsigned short v = xs[(32 + i) * kXsStride + c];
+                vals[o++] = v;
+                if (ngrp == 1) range.add(v);
+            }
     } else {
         const unsigned voff_other = __shfl_xor_sync(kFull, voff, 1);
 #pragma unroll
@@ -189,6 +209,7 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
             const unsigned thi = t ? hi1 : hi0, tlo = t ? lo1 : lo0, y = t ? y1 : y0;
             const unsigned long long bm = (static_cast<unsigned long long>(thi) << 32) | tlo;
             const unsigned off = (hh == t) ? voff : voff_other;
+            TileRange part;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int cidx = 2 * k + hh;                        // chunk inside the tile
@@ -197,29 +218,41 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const unsigned word = w[16 * t + 4 * k + (e >> 1)];
-                    if ((flags >> (7 - e)) & 1u) vals[o++] = static_cast<unsigned short>((e & 1) ? (word >> 16) : word);
+                    if ((flags >> (7 - e)) & 1u) {
+                        const unsigned short v = static_cast<unsigned short>((e & 1) ? (word >> 16) : word);
+                        vals[o++] = v;
+                        if (ngrp == 1) part.add(v);
+                    }
                 }
+            }
+            if (ngrp == 1) {   // the tile's chunks are split over the pair
+                const unsigned mine = __half_as_ushort(part.lo) | (static_cast<unsigned>(__half_as_ushort(part.hi)) << 16);
+                const unsigned other = __shfl_xor_sync(kFull, mine, 1);
+                part.lo = __hmin(part.lo, __ushort_as_half(static_cast<unsigned short>(other & 0xffffu)));
+                part.hi = __hmax(part.hi, __ushort_as_half(static_cast<unsigned short>(other >> 16)));
+                if (hh == t) range = part;
             }
         }
     }
     __syncthreads();
 
-    // ---- per tile: min / max of every group -> scale, zero (fp32 arithmetic, stored fp16).  One thread per
-    // tile; dealing the values out evenly with shared-memory min / max on ordered keys measured slower.
+    // ---- per tile: range of every group -> scale, zero (fp32 arithmetic, stored fp16)
     const int64_t gtile = p.tile_start + static_cast<int64_t>(b) * kTilesPerBlock + tile;
     const int64_t mi = h * p.meta_hs + gtile;
     {
-        float mn0 = INFINITY, mx0 = -INFINITY, mn1 = INFINITY, mx1 = -INFINITY;
-        const int n0 = (ngrp == 2 && cnt > 32) ? 32 : cnt;
-        for (int k = 0; k < n0; ++k) {
-            const float f = __half2float(__ushort_as_half(vals[voff + k]));
-            mn0 = fminf(mn0, f);
-            mx0 = fmaxf(mx0, f);
-        }
-        for (int k = n0; k < cnt; ++k) {
-            const float f = __half2float(__ushort_as_half(vals[voff + k]));
-            mn1 = fminf(mn1, f);
-            mx1 = fmaxf(mx1, f);
+        float mn0 = __half2float(range.lo), mx0 = __half2float(range.hi), mn1 = INFINITY, mx1 = -INFINITY;
+        if (ngrp == 2) {
+            const int n0 = cnt > 32 ? 32 : cnt;
+            for (int k = 0; k < n0; ++k) {
+                const float f = __half2float(__ushort_as_half(vals[voff + k]));
+                mn0 = fminf(mn0, f);
+                mx0 = fmaxf(mx0, f);
+            }
+            for (int k = n0; k < cnt; ++k) {
+                const float f = __half2float(__ushort_as_half(vals[voff + k]));
+                mn1 = fminf(mn1, f);
+                mx1 = fmaxf(mx1, f);
+            }
         }
         const GroupQ g0 = make_group(mn0, mx0, cnt > 0, maxq, &p.scales[mi * ngrp], &p.zeros[mi * ngrp]);
         GroupQ g1;
@@ -240,22 +273,34 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
 #pragma unroll
             for (int step = 64; step; step >>= 1)
                 if (t + step < 128 && s_voff[t + step] <= run0) t += step;
-            unsigned base_t = s_voff[t], next = s_voff[t + 1];
+            unsigned base_t = s_voff[t], next = s_voff[t + 1], wbase = s_woff[t];
+            float4 par = s_par[t];
+            unsigned cur = 0xffffffffu, acc = 0;   // word being filled; a run meets a word once, so one atomic each
             for (unsigned i = run0; i < run1; ++i) {
-                while (i >= next) {   // also skips empty tiles
-                    ++t;
-                    base_t = next;
-                    next = s_voff[t + 1];
+                if (i >= next) {
+                    do {   // also skips empty tiles
+                        ++t;
+                        base_t = next;
+                        next = s_voff[t + 1];
+                    } while (i >= next);
+                    wbase = s_woff[t];
+                    par = s_par[t];
                 }
                 const unsigned k = i - base_t;
-                const float4 par = s_par[t];
                 const bool g1 = (ngrp == 2 && k >= 32u);
                 const float scale = g1 ? par.z : par.x, zero = g1 ? par.w : par.y;
                 const float f = __half2float(__ushort_as_half(vals[i]));
                 float q = __fadd_rn(floorf(__fadd_rn(__fdiv_rn(f, scale), 0.5f)), zero);
                 q = fminf(fmaxf(q, 0.f), static_cast<float>(maxq));
-                atomicOr(&words[s_woff[t] + k / cap], static_cast<unsigned>(q) << ((k % cap) * p.bits));
+                const unsigned word = wbase + k / cap;
+                if (word != cur) {
+                    if (acc) atomicOr(&words[cur], acc);
+                    cur = word;
+                    acc = 0;
+                }
+                acc |= static_cast<unsigned>(q) << ((k % cap) * BITS);
             }
+            if (acc) atomicOr(&words[cur], acc);
         }
     }
 
@@ -288,6 +333,15 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
         return;
     }
     for (unsigned i = tid; i < total; i += 128) p.packed[blk_start + i] = words[i];
+}
+
+template <int KIND>
+static void launch_compress_quant(const QuantParams& p, int bits, int group, cudaStream_t s) {
+    const unsigned grid = static_cast<unsigned>(p.n_heads) * static_cast<unsigned>(p.nblk);
+    if (bits == 2 && group == 64) compress_quant_kernel<KIND, 2, 64><<<grid, 128, 0, s>>>(p);
+    else if (bits == 2) compress_quant_kernel<KIND, 2, 32><<<grid, 128, 0, s>>>(p);
+    else if (group == 64) compress_quant_kernel<KIND, 4, 64><<<grid, 128, 0, s>>>(p);
+    else compress_quant_kernel<KIND, 4, 32><<<grid, 128, 0, s>>>(p);
 }
 
 // arena mode: head_tail[h] += words appended (separate tiny launch so that no block reads a moved tail)
@@ -336,8 +390,6 @@ extern "C" int mfar_compress_quant(const void* x, int64_t x_head_stride, int64_t
     p.n_heads = n_heads;
     p.nblk = nblk;
     p.rank = prune_rank;
-    p.bits = bits;
-    p.group = group;
     p.bmp = reinterpret_cast<unsigned long long*>(bitmaps);
     p.tile_off = tile_offsets;
     p.counts = counts;
@@ -356,11 +408,10 @@ extern "C" int mfar_compress_quant(const void* x, int64_t x_head_stride, int64_t
     p.state = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 16);
     p.dev_status = dev_status;
 
-    const unsigned grid = static_cast<unsigned>(n_heads) * static_cast<unsigned>(nblk);
     if (kind == MFAR_KIND_KEY)
-        compress_quant_kernel<MFAR_KIND_KEY><<<grid, 128, 0, s>>>(p);
+        launch_compress_quant<MFAR_KIND_KEY>(p, bits, group, s);
     else
-        compress_quant_kernel<MFAR_KIND_VALUE><<<grid, 128, 0, s>>>(p);
+        launch_compress_quant<MFAR_KIND_VALUE>(p, bits, group, s);
     int r = launch_status();
     if (r) return r;
     if (packed_head_stride > 0) {
