@@ -14,7 +14,8 @@
 //      loaded them; K: down the columns of the raw block in shared memory) and leave with
 //      128-bit coalesced stores.
 // CTAs take (head, block) from an atomic ticket, head-major, so every predecessor a
-// look-back waits for has already started; the wait is bounded all the same.
+// look-back waits for has already started; the wait is bounded all the same.  Short inputs
+// (up to 8 blocks per head) run a cluster per head instead and exchange the totals directly.
 #include "compress_common.cuh"
 
 namespace mfar {
@@ -45,7 +46,7 @@ struct CompressParams {
     unsigned* max_block;           // optional: running max of packed halves per block
 };
 
-template <int KIND>
+template <int KIND, bool CLUSTER>
 __global__ void __launch_bounds__(128, KIND == MFAR_KIND_KEY ? kCompressMinCtasKey : kCompressMinCtasValue) compress_kernel(CompressParams p) {
     __shared__ __align__(16) unsigned short ps[64 * 128];                                       // packed values, final order
     __shared__ __align__(16) unsigned short xs[KIND == MFAR_KIND_KEY ? 64 * kXsStride : 8];     // K: the raw block
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(128, KIND == MFAR_KIND_KEY ? kCompressMinCtasK
     __shared__ unsigned s_warp[4][2];
     __shared__ unsigned s_ticket;
     __shared__ long long s_excl;
+    __shared__ unsigned s_totals[kClusterBlocks];
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -62,10 +64,15 @@ __global__ void __launch_bounds__(128, KIND == MFAR_KIND_KEY ? kCompressMinCtasK
     // (head, block) pairs come from an atomic ticket, fetched when the CTA is ready to start on it: blocks
     // then start in ticket order, and a look-back never waits for a predecessor that has not begun.
     {
-        if (tid == 0) s_ticket = atomicAdd(p.ticket, 1u);
-        __syncthreads();
-        const unsigned ticket = s_ticket;
-        if (ticket >= n_blocks) return;
+        unsigned ticket = blockIdx.x;
+        if (CLUSTER) {
+            cluster_open();
+        } else {
+            if (tid == 0) s_ticket = atomicAdd(p.ticket, 1u);
+            __syncthreads();
+            ticket = s_ticket;
+            if (ticket >= n_blocks) return;
+        }
         const int h = static_cast<int>(ticket / static_cast<unsigned>(p.nblk));
         const int b = static_cast<int>(ticket % static_cast<unsigned>(p.nblk));
 
@@ -152,7 +159,10 @@ __global__ void __launch_bounds__(128, KIND == MFAR_KIND_KEY ? kCompressMinCtasK
         }
         const unsigned excl_tile = incl - pad;
         unsigned long long* chain = p.state + static_cast<int64_t>(h) * p.nblk;
-        if (tid == 0) lookback_announce(chain, b, 0, total);
+        if (CLUSTER)
+            cluster_announce(s_totals, b, p.nblk, total);
+        else if (tid == 0)
+            lookback_announce(chain, b, 0, total);
 
         // ---- 5: pack in shared memory in final order (needs no global offset yet)
         if (KIND == MFAR_KIND_KEY) {
@@ -194,17 +204,24 @@ __global__ void __launch_bounds__(128, KIND == MFAR_KIND_KEY ? kCompressMinCtasK
 
         // ---- 4b: start of this block inside its head (decoupled look-back, warp 0; the predecessors
         // announced their totals a pack phase ago)
-        if (warp == 0) {
-            const long long e = lookback_exclusive(chain, b, 0, total, p.err, p.dev_status, false);
-            if (lane == 0) s_excl = e;
+        long long excl_blocks;
+        if (CLUSTER) {
+            excl_blocks = cluster_exclusive(s_totals, b);
+            __syncthreads();
+        } else {
+            if (warp == 0) {
+                const long long e = lookback_exclusive(chain, b, 0, total, p.err, p.dev_status, false);
+                if (lane == 0) s_excl = e;
+            }
+            __syncthreads();
+            excl_blocks = s_excl;
+            if (excl_blocks < 0) return;
         }
-        __syncthreads();
-        if (s_excl < 0) return;
 
         const int64_t tile0 = p.tile_start + static_cast<int64_t>(b) * kTilesPerBlock;
         int* acc = p.acc + h * p.acc_hs;
         const long long base = (p.tile_start > 0) ? static_cast<long long>(acc[p.tile_start]) : 0ll;
-        const long long blk_start = base + s_excl;  // uint32 units inside the head
+        const long long blk_start = base + excl_blocks;  // uint32 units inside the head
 
         p.bmp[h * p.bmp_hs + tile0 + tile] = (static_cast<unsigned long long>(hi) << 32) | lo;
         acc[tile0 + tile + 1] = static_cast<int>(blk_start + incl);
@@ -316,7 +333,10 @@ extern "C" int mfar_compress_fp16(const void* x, int64_t x_head_stride, int64_t 
     if (static_cast<int64_t>(n_heads) * nblk > 0x7fffffffll) return MFAR_ERR_LIMIT;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(scratch, 0, need, s) != cudaSuccess) return MFAR_ERR_LAUNCH;
+    // a cluster per head up to the portable cluster size: 256 heads x 256 tokens of K and of V
+    // take 33.3 us against 39.0 us with the look-back (a memset, tickets and polls less)
+    const bool cluster = nblk <= kClusterBlocks;
+    if (!cluster && cudaMemsetAsync(scratch, 0, need, s) != cudaSuccess) return MFAR_ERR_LAUNCH;
 
     CompressParams p;
     p.x = static_cast<const __half*>(x);
@@ -344,10 +364,13 @@ extern "C" int mfar_compress_fp16(const void* x, int64_t x_head_stride, int64_t 
 
     const unsigned n_blocks = static_cast<unsigned>(n_heads) * static_cast<unsigned>(nblk);
     const unsigned grid = n_blocks;
+    if (cluster)
+        return kind == MFAR_KIND_KEY ? launch_clusters(compress_kernel<MFAR_KIND_KEY, true>, p, grid, nblk, s)
+                                     : launch_clusters(compress_kernel<MFAR_KIND_VALUE, true>, p, grid, nblk, s);
     if (kind == MFAR_KIND_KEY)
-        compress_kernel<MFAR_KIND_KEY><<<grid, 128, 0, s>>>(p);
+        compress_kernel<MFAR_KIND_KEY, false><<<grid, 128, 0, s>>>(p);
     else
-        compress_kernel<MFAR_KIND_VALUE><<<grid, 128, 0, s>>>(p);
+        compress_kernel<MFAR_KIND_VALUE, false><<<grid, 128, 0, s>>>(p);
     return launch_status();
 }
 

@@ -191,4 +191,45 @@ __device__ __forceinline__ long long lookback_exclusive(unsigned long long* st, 
     return failed ? -1ll : excl;
 }
 
+// Chains of at most kClusterBlocks blocks (a decode append is 4) run as one thread-block cluster per head: the blocks
+// hand their totals to each other through distributed shared memory, so there is no ticket, no status word to poll and no
+// scratch to clear beforehand.  cluster_open .. cluster_announce .. cluster_exclusive, called by all threads of the CTA in
+// this order; work in between hides the two cluster barriers.
+constexpr int kClusterBlocks = 8;   // the portable cluster size
+
+__device__ __forceinline__ void cluster_open() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+// totals[b] of every CTA of the cluster (nblk of them) receives this block's total; thread r writes to CTA r
+__device__ __forceinline__ void cluster_announce(unsigned* totals, int b, int nblk, unsigned total) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA has started: its shared memory exists
+    if (static_cast<int>(threadIdx.x) < nblk) {
+        unsigned remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(totals + b)), "r"(threadIdx.x));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(total) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+// sum of the totals before block b; nobody writes to this CTA any more when it returns
+__device__ __forceinline__ unsigned cluster_exclusive(const unsigned* totals, int b) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    unsigned excl = 0;
+    for (int i = 0; i < b; ++i) excl += totals[i];
+    return excl;
+}
+
+// launches kernel(p) on n_heads * nblk CTAs of 128 threads, in clusters of nblk
+template <typename Params>
+inline int launch_clusters(void (*kernel)(Params), const Params& p, unsigned grid, int nblk, cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(128);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(nblk);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? MFAR_OK : MFAR_ERR_LAUNCH;
+}
+
 }  // namespace mfar

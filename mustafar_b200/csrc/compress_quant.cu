@@ -70,7 +70,7 @@ struct TileRange {
     }
 };
 
-template <int KIND, int BITS, int GROUP>
+template <int KIND, int BITS, int GROUP, bool CLUSTER>
 __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
     constexpr int maxq = (1 << BITS) - 1;
     constexpr int cap = 32 / BITS;             // codes per word
@@ -85,15 +85,24 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
     __shared__ unsigned s_warp[4][2];
     __shared__ unsigned s_ticket;
     __shared__ long long s_excl;
+    __shared__ unsigned s_totals[kClusterBlocks];
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int r = tid >> 1, hh = tid & 1;    // row of the block and member of the pair that owns it
-    if (tid == 0) s_ticket = atomicAdd(p.ticket, 1u);
-    __syncthreads();
-    const int h = static_cast<int>(s_ticket) / p.nblk;
-    const int b = static_cast<int>(s_ticket) % p.nblk;
-    if (h >= p.n_heads) return;
+    unsigned ticket = blockIdx.x;
+    if (CLUSTER) {
+        cluster_open();
+    } else {
+        if (tid == 0) s_ticket = atomicAdd(p.ticket, 1u);
+        __syncthreads();
+        ticket = s_ticket;
+    }
+    const int h = static_cast<int>(ticket / static_cast<unsigned>(p.nblk));
+    const int b = static_cast<int>(ticket % static_cast<unsigned>(p.nblk));
+    if (h >= p.n_heads) return;   // (never in a cluster launch: its grid is exact)
+    // arena mode: where the head's stream ended before this call
+    const long long old_tail = (p.packed_hs != 0 && p.head_tail) ? p.head_tail[h] : 0;
 
     // ---- the pair loads one row, selects the threshold, ends up with one "kept and nonzero" flag per element
     uint4 v[8];
@@ -180,7 +189,10 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
     const bool compact = p.packed_hs == 0;
     const int pos = h * p.nblk + b;
     const int chain_first = compact ? 0 : h * p.nblk;
-    if (tid == 0) lookback_announce(p.state, pos, chain_first, total);
+    if (CLUSTER)
+        cluster_announce(s_totals, b, p.nblk, total);
+    else if (tid == 0)
+        lookback_announce(p.state, pos, chain_first, total);
 
     // ---- kept values into vals, tile order (K: down the columns of the raw block; V: from the registers).  With one
     // parameter group per tile its range is taken on the way; with two, the rank of a value decides its group (below)
@@ -304,25 +316,31 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
         }
     }
 
-    if (warp == 0) {
-        const long long e = lookback_exclusive(p.state, pos, chain_first, total, p.err, p.dev_status, false);
-        if (lane == 0) s_excl = e;
+    long long excl_blocks;
+    if (CLUSTER) {
+        excl_blocks = cluster_exclusive(s_totals, b);
+        __syncthreads();
+    } else {
+        if (warp == 0) {
+            const long long e = lookback_exclusive(p.state, pos, chain_first, total, p.err, p.dev_status, false);
+            if (lane == 0) s_excl = e;
+        }
+        __syncthreads();
+        excl_blocks = s_excl;
+        if (excl_blocks < 0) return;
     }
-    __syncthreads();
-    if (s_excl < 0) return;
 
     long long blk_start;   // uint32 offset in the flat packed buffer
     long long limit;
     if (compact) {
-        blk_start = s_excl;
+        blk_start = excl_blocks;
         limit = p.packed_cap;
         if (p.head_tail && b == p.nblk - 1 && tid == 0) p.head_tail[h] = static_cast<int>(blk_start + total);
     } else {
-        // (in arena mode head_tail[h] is bumped by quant_bump_tails after this kernel, so every
-        // block of the head reads the same, old, tail)
-        const long long tail = p.head_tail ? p.head_tail[h] : 0;
-        blk_start = h * p.packed_hs + tail + s_excl;
+        blk_start = h * p.packed_hs + old_tail + excl_blocks;
         limit = h * p.packed_hs + p.packed_cap;
+        // the cluster's CTAs have all read the old tail; otherwise quant_bump_tails moves it after this kernel
+        if (CLUSTER && b == p.nblk - 1 && tid == 0) p.head_tail[h] = static_cast<int>(old_tail + excl_blocks + total);
     }
     p.bmp[h * p.bmp_hs + gtile] = (static_cast<unsigned long long>(hi) << 32) | lo;
     p.tile_off[mi] = static_cast<int>(blk_start + woff);
@@ -335,13 +353,19 @@ __global__ void __launch_bounds__(128) compress_quant_kernel(QuantParams p) {
     for (unsigned i = tid; i < total; i += 128) p.packed[blk_start + i] = words[i];
 }
 
-template <int KIND>
-static void launch_compress_quant(const QuantParams& p, int bits, int group, cudaStream_t s) {
+template <int KIND, int BITS, int GROUP>
+static int launch_compress_quant(const QuantParams& p, bool cluster, cudaStream_t s) {
     const unsigned grid = static_cast<unsigned>(p.n_heads) * static_cast<unsigned>(p.nblk);
-    if (bits == 2 && group == 64) compress_quant_kernel<KIND, 2, 64><<<grid, 128, 0, s>>>(p);
-    else if (bits == 2) compress_quant_kernel<KIND, 2, 32><<<grid, 128, 0, s>>>(p);
-    else if (group == 64) compress_quant_kernel<KIND, 4, 64><<<grid, 128, 0, s>>>(p);
-    else compress_quant_kernel<KIND, 4, 32><<<grid, 128, 0, s>>>(p);
+    if (cluster) return launch_clusters(compress_quant_kernel<KIND, BITS, GROUP, true>, p, grid, p.nblk, s);
+    compress_quant_kernel<KIND, BITS, GROUP, false><<<grid, 128, 0, s>>>(p);
+    return launch_status();
+}
+
+template <int KIND>
+static int dispatch_compress_quant(const QuantParams& p, int bits, int group, bool cluster, cudaStream_t s) {
+    if (bits == 2)
+        return group == 64 ? launch_compress_quant<KIND, 2, 64>(p, cluster, s) : launch_compress_quant<KIND, 2, 32>(p, cluster, s);
+    return group == 64 ? launch_compress_quant<KIND, 4, 64>(p, cluster, s) : launch_compress_quant<KIND, 4, 32>(p, cluster, s);
 }
 
 // arena mode: head_tail[h] += words appended (separate tiny launch so that no block reads a moved tail)
@@ -379,7 +403,9 @@ extern "C" int mfar_compress_quant(const void* x, int64_t x_head_stride, int64_t
     if (static_cast<int64_t>(n_heads) * nblk > 0x7fffffffll) return MFAR_ERR_LIMIT;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(scratch, 0, need, s) != cudaSuccess) return MFAR_ERR_LAUNCH;
+    // a cluster per head up to the portable cluster size (one chain over all heads stays with the look-back)
+    const bool cluster = nblk <= kClusterBlocks && (packed_head_stride > 0 || n_heads == 1);
+    if (!cluster && cudaMemsetAsync(scratch, 0, need, s) != cudaSuccess) return MFAR_ERR_LAUNCH;
 
     QuantParams p;
     p.x = static_cast<const __half*>(x);
@@ -408,13 +434,10 @@ extern "C" int mfar_compress_quant(const void* x, int64_t x_head_stride, int64_t
     p.state = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 16);
     p.dev_status = dev_status;
 
-    if (kind == MFAR_KIND_KEY)
-        launch_compress_quant<MFAR_KIND_KEY>(p, bits, group, s);
-    else
-        launch_compress_quant<MFAR_KIND_VALUE>(p, bits, group, s);
-    int r = launch_status();
+    int r = kind == MFAR_KIND_KEY ? dispatch_compress_quant<MFAR_KIND_KEY>(p, bits, group, cluster, s)
+                                  : dispatch_compress_quant<MFAR_KIND_VALUE>(p, bits, group, cluster, s);
     if (r) return r;
-    if (packed_head_stride > 0) {
+    if (packed_head_stride > 0 && !cluster) {
         quant_bump_tails<<<(n_heads + 127) / 128, 128, 0, s>>>(p.state, nblk, n_heads, head_tail);
         r = launch_status();
     }
