@@ -48,6 +48,14 @@ SIGNATURES = {
                                      _vp, _i64, _vp, _vp]),
     "mfar_value_output_quant": (_i32, [_vp, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _i32, _i32, _i32,
                                        _vp, _i64, _vp, _sz, _i32, _vp, _vp]),
+    "mfar_key_scores_rows_fp16": (_i32, [_vp, _i64, _i32, _i32, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i32,
+                                         _vp, _i64, _i32, _i64, _i32, _vp, _vp]),
+    "mfar_value_output_rows_fp16": (_i32, [_vp, _i64, _i32, _i32, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i32,
+                                           _vp, _i64, _i32, _i64, _vp, _sz, _i32, _i32, _vp, _vp]),
+    "mfar_key_scores_rows_quant": (_i32, [_vp, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _i32, _i32, _i32,
+                                          _vp, _i64, _i32, _i64, _vp, _vp]),
+    "mfar_value_output_rows_quant": (_i32, [_vp, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _i32, _i32, _i32,
+                                            _vp, _i64, _i32, _i64, _vp, _sz, _i32, _vp, _vp]),
     "mfar_decode_attention_quant": (_i32, [_vp, _i64, _i32, _i32,
                                            _vp, _vp, _vp, _vp, _vp, _i64,
                                            _vp, _vp, _vp, _vp, _vp, _i64,

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
                 for (int e = 0; e < 4; ++e) dv[hf][f][j][e] = 0.f;
 
     bool timed_out = false;
+    int done = 0;   // blocks finished
     for (int i = 0; i < nb; ++i) {
         const unsigned char* st = smem + lay.stages + static_cast<size_t>(i % kStages) * stg;
         const uint2* bm_s = reinterpret_cast<const uint2*>(st);
@@ -134,6 +135,9 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
         const unsigned* of = off + (i & 1) * 128;
 
         if (i + 1 < nb) fetch_offsets(i + 1);
+        if (MODE == MODE_KEY && p.rows > 1)
+            zero_score_rows<G>(p.s_out + static_cast<int64_t>(h) * G * p.s_stride + static_cast<int64_t>(blk0 + i) * 64, p.s_stride,
+                               p.rows, p.row_stride, 1);
         unsigned pp[2] = {0u, 0u};   // VALUE: probabilities of tokens warp*16 + 8*vg + 2*cp, + 1
         if (MODE == MODE_VALUE && prow) {
             pp[0] = ldg_nc_u32(prow + static_cast<int64_t>(i) * 64);
@@ -141,6 +145,7 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
         }
         if (!mbar_wait(&bars[i % kStages], (i / kStages) & 1)) timed_out = true;
         if (__syncthreads_or(timed_out)) { timed_out = true; break; }   // also publishes the stage hand-off below
+        done = i + 1;
         if (tid == 0 && i + kStages - 1 < nb) issue(i + kStages - 1);
 
         auto expand2 = [&](int tile, unsigned (&r1)[4], unsigned (&r2)[4]) {
@@ -203,6 +208,11 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
 
     if (timed_out) {
         if (tid == 0 && p.dev_status) atomicOr(p.dev_status, MFAR_DEV_TIMEOUT);
+        if (MODE == MODE_KEY && p.rows > 1) {   // the padded result stays defined: zero from the lost block on
+            for (int i = done; i < nb; ++i)
+                zero_score_rows<G>(p.s_out + static_cast<int64_t>(h) * G * p.s_stride + static_cast<int64_t>(blk0 + i) * 64, p.s_stride,
+                                   p.rows, p.row_stride, 0);
+        }
         return;
     }
     if (MODE == MODE_KEY) return;
@@ -234,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
 // Merges the split partials of one q head: out = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M)
 // (normalise = 1) or the plain sum of O_s (normalise = 0).  One CTA per q head, 128 threads.
 __global__ void __launch_bounds__(128) combine_kernel(const float* ws, int nrec, int G, int normalise,
-                                                      __half* out, int64_t out_stride) {
+                                                      __half* out, int64_t out_stride, int rows, int64_t row_stride) {
     // weight of each record, computed once per CTA (records in chunks of 128), then every thread sums
     // its channel over the records with independent, unrolled loads
     __shared__ float w_s[128];
@@ -283,6 +293,7 @@ __global__ void __launch_bounds__(128) combine_kernel(const float* ws, int nrec,
     }
     if (normalise) o = (l > 0.f) ? o / l : 0.f;
     out[bq * out_stride + c] = __float2half_rn(o);
+    for (int r = 1; r < rows; ++r) out[bq * out_stride + r * row_stride + c] = __float2half_rn(0.f);
 }
 
 // ---------------------------------------------------------------------------- host side
@@ -328,8 +339,8 @@ static int check_sparse(const void* bmp, const void* acc, const void* nz, int64_
 }
 
 int launch_combine(const float* ws, int nrec, int G, int normalise, void* out, int64_t out_stride, int n_q_heads,
-                   cudaStream_t s) {
-    combine_kernel<<<n_q_heads, 128, 0, s>>>(ws, nrec, G, normalise, static_cast<__half*>(out), out_stride);
+                   cudaStream_t s, int rows, int64_t row_stride) {
+    combine_kernel<<<n_q_heads, 128, 0, s>>>(ws, nrec, G, normalise, static_cast<__half*>(out), out_stride, rows, row_stride);
     return launch_status();
 }
 
@@ -460,16 +471,18 @@ extern "C" int mfar_decode_attention_fp16_dyn(
                                       workspace, workspace_bytes, nsplit, stage_halves, dev_status, stream);
 }
 
-extern "C" int mfar_key_scores_fp16(const void* q, int64_t q_stride, int n_kv_heads, int group,
+extern "C" int mfar_key_scores_rows_fp16(const void* q, int64_t q_stride, int n_kv_heads, int group,
                                     const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* accum,
                                     int64_t acc_head_stride, const void* nz, const int32_t* nz_offset,
                                     int64_t nz_head_stride, int64_t nz_extent, int n_tokens, void* scores,
-                                    int64_t scores_stride, int stage_halves, uint32_t* dev_status, void* stream) {
+                                    int64_t scores_stride, int rows, int64_t row_stride, int stage_halves, uint32_t* dev_status, void* stream) {
+    if (rows < 1) return MFAR_ERR_ARG;
     if (n_kv_heads <= 0 || group <= 0 || n_tokens < 0 || (n_tokens % 64) || nz_extent < 0) return MFAR_ERR_ARG;
     if (group != 1 && group != 2 && group != 4 && group != 8) return MFAR_ERR_ARG;
     if (n_tokens == 0) return MFAR_OK;
     if (!q || !scores) return MFAR_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(scores) & 3) || (scores_stride & 1)) return MFAR_ERR_ALIGN;
+    if (rows > 1 && ((reinterpret_cast<uintptr_t>(scores) & 15) || (scores_stride & 7) || (row_stride & 7))) return MFAR_ERR_ALIGN;
     int r = check_sparse(bitmaps, accum, nz, bmp_head_stride, nz_head_stride);
     if (r) return r;
     DecodeParams p{};
@@ -489,17 +502,30 @@ extern "C" int mfar_key_scores_fp16(const void* q, int64_t q_stride, int n_kv_he
     p.cap = pick_cap(stage_halves);
     p.s_out = static_cast<__half*>(scores);
     p.s_stride = scores_stride;
+    p.rows = rows;
+    p.row_stride = row_stride;
     p.dev_status = dev_status;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return dispatch_spmv<MODE_KEY>(p, group, n_kv_heads, p.nsplit, s);
 }
 
-extern "C" int mfar_value_output_fp16(const void* probs, int64_t probs_stride, int n_kv_heads, int group,
+extern "C" int mfar_key_scores_fp16(const void* q, int64_t q_stride, int n_kv_heads, int group,
+                                    const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* accum,
+                                    int64_t acc_head_stride, const void* nz, const int32_t* nz_offset,
+                                    int64_t nz_head_stride, int64_t nz_extent, int n_tokens, void* scores,
+                                    int64_t scores_stride, int stage_halves, uint32_t* dev_status, void* stream) {
+    return mfar_key_scores_rows_fp16(q, q_stride, n_kv_heads, group, bitmaps, bmp_head_stride, accum, acc_head_stride, nz,
+                                     nz_offset, nz_head_stride, nz_extent, n_tokens, scores, scores_stride, 1, 0, stage_halves,
+                                     dev_status, stream);
+}
+
+extern "C" int mfar_value_output_rows_fp16(const void* probs, int64_t probs_stride, int n_kv_heads, int group,
                                       const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* accum,
                                       int64_t acc_head_stride, const void* nz, const int32_t* nz_offset,
                                       int64_t nz_head_stride, int64_t nz_extent, int n_tokens, void* out,
-                                      int64_t out_stride, void* workspace, size_t workspace_bytes, int nsplit,
+                                      int64_t out_stride, int rows, int64_t row_stride, void* workspace, size_t workspace_bytes, int nsplit,
                                       int stage_halves, uint32_t* dev_status, void* stream) {
+    if (rows < 1) return MFAR_ERR_ARG;
     if (n_kv_heads <= 0 || group <= 0 || n_tokens <= 0 || (n_tokens % 64) || nz_extent < 0) return MFAR_ERR_ARG;
     if (group != 1 && group != 2 && group != 4 && group != 8) return MFAR_ERR_ARG;
     if (!probs || !out || !workspace) return MFAR_ERR_ARG;
@@ -526,5 +552,16 @@ extern "C" int mfar_value_output_fp16(const void* probs, int64_t probs_stride, i
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     r = dispatch_spmv<MODE_VALUE>(p, group, n_kv_heads, ns, s);
     if (r) return r;
-    return launch_combine(p.ws, ns, group, 0, out, out_stride, n_kv_heads * group, s);
+    return launch_combine(p.ws, ns, group, 0, out, out_stride, n_kv_heads * group, s, rows, row_stride);
+}
+
+extern "C" int mfar_value_output_fp16(const void* probs, int64_t probs_stride, int n_kv_heads, int group,
+                                      const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* accum,
+                                      int64_t acc_head_stride, const void* nz, const int32_t* nz_offset,
+                                      int64_t nz_head_stride, int64_t nz_extent, int n_tokens, void* out,
+                                      int64_t out_stride, void* workspace, size_t workspace_bytes, int nsplit,
+                                      int stage_halves, uint32_t* dev_status, void* stream) {
+    return mfar_value_output_rows_fp16(probs, probs_stride, n_kv_heads, group, bitmaps, bmp_head_stride, accum, acc_head_stride,
+                                       nz, nz_offset, nz_head_stride, nz_extent, n_tokens, out, out_stride, 1, 0, workspace,
+                                       workspace_bytes, nsplit, stage_halves, dev_status, stream);
 }

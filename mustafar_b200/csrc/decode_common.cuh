@@ -220,6 +220,8 @@ struct DecodeParams {
     int nrec;              // partial records per kv head in ws
     __half* s_out;         // MODE_KEY  : [Bq][s_stride]
     int64_t s_stride;
+    int rows;              // MODE_KEY  : result rows per query head; row 0 is the product, the rest is zero-filled
+    int64_t row_stride;
     const __half* p_in;    // MODE_VALUE: [Bq][p_stride]
     int64_t p_stride;
     unsigned* dev_status;
@@ -254,8 +256,20 @@ int launch_decode_attn(const DecodeParams& p, int G, int n_kv_heads, int grid_x,
 int launch_decode_attn_quant(const DecodeParams& p, int G, int bits, bool group32, int n_kv_heads, int grid_x,
                              cudaStream_t s);
 // merge of the split-KV records (normalise = 1) or plain sum (normalise = 0), one CTA per q head
+// (rows > 1: rows 1.. of every head, row_stride apart, are zero-filled)
 int launch_combine(const float* ws, int nrec, int G, int normalise, void* out, int64_t out_stride, int n_q_heads,
-                   cudaStream_t s);
+                   cudaStream_t s, int rows = 1, int64_t row_stride = 0);
+
+// Zero-fills rows 1 .. rows - 1 (row 0 too with `first` = 0) of one 64-token block's scores for G query heads, 16 bytes a
+// store: a separate fill of the padded result would move it through memory a second time.
+template <int G>
+__device__ __forceinline__ void zero_score_rows(__half* block, int64_t head_stride, int rows, int64_t row_stride, int first) {
+    const int per_head = (rows - first) * 8;
+    for (int i = threadIdx.x; i < G * per_head; i += blockDim.x) {
+        const int g = i / per_head, r = first + (i % per_head) / 8;
+        *reinterpret_cast<uint4*>(block + g * head_stride + r * row_stride + 8 * (i & 7)) = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
 // Split count of the 64-token-block decode kernels.  The grid is n_kv_heads * ns CTAs of bps = ceil(nblk / ns) blocks.
 // The cost of a candidate follows a model fitted to a measured sweep of ns over batch 1..64 and
 // 4k..32k tokens on a B200 (all times in units of one block on an otherwise idle SM, ~2 us):

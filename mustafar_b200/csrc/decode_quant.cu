@@ -34,6 +34,8 @@ struct QDecodeParams {
     float* ws;
     __half* s_out;
     int64_t s_stride;
+    int rows;              // result rows per query head (MODE_KEY); row 0 is the product, the rest is zero-filled
+    int64_t row_stride;
     const __half* p_in;
     int64_t p_stride;
     unsigned* dev_status;
@@ -181,6 +183,9 @@ __global__ void __launch_bounds__(kQThreads, 4) decode_quant_kernel(QDecodeParam
     constexpr int kHeadsPerWarp = (G + kQWarps - 1) / kQWarps;
 
     for (int i = 0; i < nb; ++i) {
+        if (MODE == MODE_KEY && p.rows > 1)
+            zero_score_rows<G>(p.s_out + static_cast<int64_t>(hq) * G * p.s_stride + static_cast<int64_t>(blk0 + i) * 64, p.s_stride,
+                               p.rows, p.row_stride, 1);
         cp_async_wait_all();
         __syncthreads();   // block i has landed for everybody; everybody is done with block i-1
         if (i + 1 < nb) {
@@ -356,15 +361,17 @@ static void q_split(int n_kv_heads, int nblk, int hint, int* ns, int* bps) {
 
 using namespace mfar;
 
-extern "C" int mfar_key_scores_quant(const void* q, int64_t q_stride, int n_kv_heads, int group,
+extern "C" int mfar_key_scores_rows_quant(const void* q, int64_t q_stride, int n_kv_heads, int group,
                                      const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* tile_offsets,
                                      const void* scales, const void* zeros, int64_t meta_head_stride,
                                      const int32_t* packed, int64_t packed_words, int n_tokens, int bits, int qgroup,
-                                     void* scores, int64_t scores_stride, uint32_t* dev_status, void* stream) {
+                                     void* scores, int64_t scores_stride, int rows, int64_t row_stride, uint32_t* dev_status, void* stream) {
+    if (rows < 1) return MFAR_ERR_ARG;
     if (n_kv_heads <= 0 || group <= 0 || n_tokens < 0 || (n_tokens % 64) || packed_words < 0) return MFAR_ERR_ARG;
     if (n_tokens == 0) return MFAR_OK;
     if (!q || !scores) return MFAR_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(scores) & 3) || (scores_stride & 1)) return MFAR_ERR_ALIGN;
+    if (rows > 1 && ((reinterpret_cast<uintptr_t>(scores) & 15) || (scores_stride & 7) || (row_stride & 7))) return MFAR_ERR_ALIGN;
     int r = check_q(bitmaps, tile_offsets, scales, zeros, packed, bits, qgroup);
     if (r) return r;
     QDecodeParams p{};
@@ -378,16 +385,29 @@ extern "C" int mfar_key_scores_quant(const void* q, int64_t q_stride, int n_kv_h
     p.group32 = qgroup == 32;
     p.s_out = static_cast<__half*>(scores);
     p.s_stride = scores_stride;
+    p.rows = rows;
+    p.row_stride = row_stride;
     p.dev_status = dev_status;
     return dispatch_q<MODE_KEY>(p, group, bits, n_kv_heads, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int mfar_value_output_quant(const void* probs, int64_t probs_stride, int n_kv_heads, int group,
+extern "C" int mfar_key_scores_quant(const void* q, int64_t q_stride, int n_kv_heads, int group,
+                                     const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* tile_offsets,
+                                     const void* scales, const void* zeros, int64_t meta_head_stride,
+                                     const int32_t* packed, int64_t packed_words, int n_tokens, int bits, int qgroup,
+                                     void* scores, int64_t scores_stride, uint32_t* dev_status, void* stream) {
+    return mfar_key_scores_rows_quant(q, q_stride, n_kv_heads, group, bitmaps, bmp_head_stride, tile_offsets, scales, zeros,
+                                      meta_head_stride, packed, packed_words, n_tokens, bits, qgroup, scores, scores_stride, 1, 0,
+                                      dev_status, stream);
+}
+
+extern "C" int mfar_value_output_rows_quant(const void* probs, int64_t probs_stride, int n_kv_heads, int group,
                                        const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* tile_offsets,
                                        const void* scales, const void* zeros, int64_t meta_head_stride,
                                        const int32_t* packed, int64_t packed_words, int n_tokens, int bits, int qgroup,
-                                       void* out, int64_t out_stride, void* workspace, size_t workspace_bytes,
+                                       void* out, int64_t out_stride, int rows, int64_t row_stride, void* workspace, size_t workspace_bytes,
                                        int nsplit, uint32_t* dev_status, void* stream) {
+    if (rows < 1) return MFAR_ERR_ARG;
     if (n_kv_heads <= 0 || group <= 0 || n_tokens <= 0 || (n_tokens % 64) || packed_words < 0) return MFAR_ERR_ARG;
     if (!probs || !out || !workspace) return MFAR_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(probs) & 3) || (probs_stride & 1)) return MFAR_ERR_ALIGN;
@@ -410,7 +430,18 @@ extern "C" int mfar_value_output_quant(const void* probs, int64_t probs_stride, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     r = dispatch_q<MODE_VALUE>(p, group, bits, n_kv_heads, s);
     if (r) return r;
-    return launch_combine(p.ws, p.nrec, group == 8 ? 4 : group, 0, out, out_stride, n_kv_heads * group, s);
+    return launch_combine(p.ws, p.nrec, group == 8 ? 4 : group, 0, out, out_stride, n_kv_heads * group, s, rows, row_stride);
+}
+
+extern "C" int mfar_value_output_quant(const void* probs, int64_t probs_stride, int n_kv_heads, int group,
+                                       const int64_t* bitmaps, int64_t bmp_head_stride, const int32_t* tile_offsets,
+                                       const void* scales, const void* zeros, int64_t meta_head_stride,
+                                       const int32_t* packed, int64_t packed_words, int n_tokens, int bits, int qgroup,
+                                       void* out, int64_t out_stride, void* workspace, size_t workspace_bytes,
+                                       int nsplit, uint32_t* dev_status, void* stream) {
+    return mfar_value_output_rows_quant(probs, probs_stride, n_kv_heads, group, bitmaps, bmp_head_stride, tile_offsets, scales,
+                                        zeros, meta_head_stride, packed, packed_words, n_tokens, bits, qgroup, out, out_stride, 1, 0,
+                                        workspace, workspace_bytes, nsplit, dev_status, stream);
 }
 
 extern "C" int mfar_decode_attention_quant(

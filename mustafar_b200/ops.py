@@ -119,14 +119,14 @@ def mustafar_key_formulation(bmp, NZ, idx, NZ_Offset, B, M_Global, K_Global, Bat
         raise RuntimeError("B must be contiguous.")
     n_kv = Batch_Size // num_key_value_groups
     tiles = M_Global * K_Global // 64
-    out = torch.zeros((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
+    out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
     st = _dev_status(B.device)
     rows = B.shape[1] if B.dim() == 3 else 1
-    r = _lib.lib().mfar_key_scores_fp16(
+    r = _lib.lib().mfar_key_scores_rows_fp16(
         B.data_ptr(), rows * K_Global, n_kv, num_key_value_groups,
         bmp.data_ptr(), tiles, idx.data_ptr(), tiles + 1, NZ.data_ptr(), NZ_Offset.data_ptr(), 0, NZ.numel(),
-        M_Global, out.data_ptr(), 8 * M_Global, 0, st.data_ptr(), _stream())
-    _lib.check(r, "mfar_key_scores_fp16")
+        M_Global, out.data_ptr(), 8 * M_Global, 8, M_Global, 0, st.data_ptr(), _stream())
+    _lib.check(r, "mfar_key_scores_rows_fp16")
     if _debug_check():
         check_device_status(B.device)
     return out
@@ -146,16 +146,16 @@ def mustafar_value_formulation(bmp, NZ, idx, NZ_Offset, B, Reduction_Workspace, 
     Bc = B if B.is_contiguous() else B.contiguous()
     n_kv = Batch_Size // num_key_value_groups
     tiles = M_Global * K_Global // 64
-    out = torch.zeros((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
+    out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
     _, nbytes = plan(n_kv, K_Global, 0, num_key_value_groups)
     ws = _workspace(B.device, nbytes)
     st = _dev_status(B.device)
     rows = Bc.shape[1] if Bc.dim() == 3 else 1
-    r = _lib.lib().mfar_value_output_fp16(
+    r = _lib.lib().mfar_value_output_rows_fp16(
         Bc.data_ptr(), rows * K_Global, n_kv, num_key_value_groups,
         bmp.data_ptr(), tiles, idx.data_ptr(), tiles + 1, NZ.data_ptr(), NZ_Offset.data_ptr(), 0, NZ.numel(),
-        K_Global, out.data_ptr(), 8 * M_Global, ws.data_ptr(), ws.numel(), 0, 0, st.data_ptr(), _stream())
-    _lib.check(r, "mfar_value_output_fp16")
+        K_Global, out.data_ptr(), 8 * M_Global, 8, M_Global, ws.data_ptr(), ws.numel(), 0, 0, st.data_ptr(), _stream())
+    _lib.check(r, "mfar_value_output_rows_fp16")
     if _debug_check():
         check_device_status(B.device)
     return out

@@ -56,14 +56,14 @@ def mustafar_key_formulation_quant(bmp, NZ_quant, tile_offsets, scales, zeros, B
         raise RuntimeError("B must be contiguous.")
     n_kv = Batch_Size // num_key_value_groups
     tiles = M_Global * K_Global // 64
-    out = torch.zeros((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
+    out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
     st = _dev_status(B.device)
     rows = B.shape[1] if B.dim() == 3 else 1
-    r = _lib.lib().mfar_key_scores_quant(
+    r = _lib.lib().mfar_key_scores_rows_quant(
         B.data_ptr(), rows * K_Global, n_kv, num_key_value_groups, bmp.data_ptr(), tiles, tile_offsets.data_ptr(),
         scales.data_ptr(), zeros.data_ptr(), tiles, NZ_quant.data_ptr(), NZ_quant.numel(), M_Global, bit,
-        _qgroup(scales, n_kv, tiles), out.data_ptr(), 8 * M_Global, st.data_ptr(), _stream())
-    _lib.check(r, "mfar_key_scores_quant")
+        _qgroup(scales, n_kv, tiles), out.data_ptr(), 8 * M_Global, 8, M_Global, st.data_ptr(), _stream())
+    _lib.check(r, "mfar_key_scores_rows_quant")
     if _debug_check():
         check_device_status(B.device)
     return out
@@ -87,11 +87,11 @@ def _value(bmp, NZ_quant, tile_offsets, scales, zeros, P, probs_stride, M_Global
     _, nbytes = plan(n_kv, K_Global, 0, groups)
     ws = _workspace(P.device, max(nbytes, 65536 + n_kv * max(1, K_Global // 64) * groups * 132 * 4))
     st = _dev_status(P.device)
-    r = _lib.lib().mfar_value_output_quant(
+    r = _lib.lib().mfar_value_output_rows_quant(
         P.data_ptr(), probs_stride, n_kv, groups, bmp.data_ptr(), tiles, tile_offsets.data_ptr(), scales.data_ptr(),
         zeros.data_ptr(), tiles, NZ_quant.data_ptr(), NZ_quant.numel(), K_Global, bit, _qgroup(scales, n_kv, tiles),
-        out.data_ptr(), out_stride, ws.data_ptr(), ws.numel(), 0, st.data_ptr(), _stream())
-    _lib.check(r, "mfar_value_output_quant")
+        out.data_ptr(), out_stride, out_stride // M_Global, M_Global, ws.data_ptr(), ws.numel(), 0, st.data_ptr(), _stream())
+    _lib.check(r, "mfar_value_output_rows_quant")
     if _debug_check():
         check_device_status(P.device)
     return out
@@ -102,7 +102,7 @@ def mustafar_value_formulation_quant(bmp, NZ_quant, tile_offsets, tile_counts, t
                                      capacity, dequant_mode=0, split_k=1, value_tile_config=0):
     """O = dequant(V~)^T p; B [Batch_Size, 8, L] (row 0 = probabilities) -> fp16 [Batch_Size, 8, 128]."""
     Bc = B if B.is_contiguous() else B.contiguous()
-    out = torch.zeros((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
+    out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
     rows = Bc.shape[1] if Bc.dim() == 3 else 1
     return _value(bmp, NZ_quant, tile_offsets, scales, zeros, Bc, rows * K_Global, M_Global, K_Global, Batch_Size,
                   num_key_value_groups, bit, capacity, out, 8 * M_Global, split_k)
