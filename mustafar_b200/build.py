@@ -1,4 +1,5 @@
-"""Builds libmustafar_b200.so (all CUDA sources of csrc/, sm_100a only) in-tree with nvcc.
+"""Builds libmustafar_b200.so (all CUDA sources of csrc/, sm_100a only) and _native.so (the CPython binding of its
+hot entry points) in-tree with nvcc.
 
     python -m mustafar_b200.build [--force] [--verbose]
 
@@ -13,12 +14,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libmustafar_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]
 
@@ -72,6 +75,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    src = os.path.join(CSRC, "native.cpp")
+    if force or not os.path.exists(NATIVE) or os.path.getmtime(NATIVE) < max(os.path.getmtime(src), hdr_t):
+        cmd = [nvcc, "-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-cudart", "none", "-o", NATIVE, src,
+               "-I", sysconfig.get_path("include"), "-L", HERE, "-l:" + os.path.basename(LIB), "-Xlinker", "-rpath=$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("the CPython binding failed to build")
     return LIB
 
 

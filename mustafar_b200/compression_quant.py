@@ -36,7 +36,7 @@ def compress_quant(x: torch.Tensor, kind: int, prune_rank: int = 0, bits: int = 
     if L:
         need = _lib.lib().mfar_compress_scratch_bytes(Bh, L)
         scratch = torch.empty(need, dtype=torch.uint8, device=dev)
-        st = _lib.lib().mfar_compress_quant(
+        st = _lib.native().mfar_compress_quant(
             x.data_ptr(), x.stride(0), x.stride(1), 0, 0, Bh, L, kind, prune_rank, bits, group,
             bitmaps.data_ptr(), T, tile_offsets.data_ptr(), counts.data_ptr(), units.data_ptr(),
             scales.data_ptr(), zeros.data_ptr(), T, 0, packed.data_ptr(), 0, worst, info.data_ptr(),
@@ -93,7 +93,7 @@ class QuantStore:
         if self._scratch is None or self._scratch.numel() < need:
             self._scratch = torch.empty(need, dtype=torch.uint8, device=self.bitmaps.device)
         T = self.tiles_cap
-        st = _lib.lib().mfar_compress_quant(
+        st = _lib.native().mfar_compress_quant(
             ptr, hs, ts, hpg, gs, self.n_heads, n, self.kind, prune_rank, self.bits, self.group,
             self.bitmaps.data_ptr(), T, self.tile_offsets.data_ptr(), self.counts.data_ptr(), self.units.data_ptr(),
             self.scales.data_ptr(), self.zeros.data_ptr(), T, 2 * self.tokens, self.packed.data_ptr(),

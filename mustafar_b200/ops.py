@@ -9,6 +9,7 @@ signatures, checks and return shapes of the reference extension
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 import os
 
@@ -38,7 +39,8 @@ def _workspace(device, nbytes: int) -> torch.Tensor:
     decode calls on several streams hands its own buffer to ``decode_attention(workspace=...)`` instead: growing
     this one while a captured graph still holds the old pointer would leave the graph writing into freed memory,
     so growth during capture is refused."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
+    index = torch._C._cuda_getDevice() if device.index is None else device.index
+    key = (device, torch._C._cuda_getCurrentRawStream(index))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         if torch.cuda.is_current_stream_capturing():
@@ -80,6 +82,15 @@ def _take_workspace(workspace, device, nbytes: int) -> torch.Tensor:
 
 
 def plan(n_kv_heads: int, n_tokens: int, window: int, group: int, nsplit: int = 0):
+    """(splits, workspace bytes) of a decode call on the current device."""
+    # without a CUDA context the library plans for a default device, which is not to be remembered
+    if not torch.cuda.is_initialized():
+        return _plan.__wrapped__(-1, n_kv_heads, n_tokens, window, group, nsplit)
+    return _plan(torch._C._cuda_getDevice(), n_kv_heads, n_tokens, window, group, nsplit)
+
+
+@functools.lru_cache(maxsize=256)
+def _plan(device_index: int, n_kv_heads: int, n_tokens: int, window: int, group: int, nsplit: int):
     ns, nbytes = C.c_int(0), C.c_size_t(0)
     _lib.check(_lib.lib().mfar_decode_plan(n_kv_heads, n_tokens, window, nsplit, C.byref(ns), C.byref(nbytes), group),
                "mfar_decode_plan")
@@ -122,7 +133,7 @@ def mustafar_key_formulation(bmp, NZ, idx, NZ_Offset, B, M_Global, K_Global, Bat
     out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
     st = _dev_status(B.device)
     rows = B.shape[1] if B.dim() == 3 else 1
-    r = _lib.lib().mfar_key_scores_rows_fp16(
+    r = _lib.native().mfar_key_scores_rows_fp16(
         B.data_ptr(), rows * K_Global, n_kv, num_key_value_groups,
         bmp.data_ptr(), tiles, idx.data_ptr(), tiles + 1, NZ.data_ptr(), NZ_Offset.data_ptr(), 0, NZ.numel(),
         M_Global, out.data_ptr(), 8 * M_Global, 8, M_Global, 0, st.data_ptr(), _stream())
@@ -151,7 +162,7 @@ def mustafar_value_formulation(bmp, NZ, idx, NZ_Offset, B, Reduction_Workspace, 
     ws = _workspace(B.device, nbytes)
     st = _dev_status(B.device)
     rows = Bc.shape[1] if Bc.dim() == 3 else 1
-    r = _lib.lib().mfar_value_output_rows_fp16(
+    r = _lib.native().mfar_value_output_rows_fp16(
         Bc.data_ptr(), rows * K_Global, n_kv, num_key_value_groups,
         bmp.data_ptr(), tiles, idx.data_ptr(), tiles + 1, NZ.data_ptr(), NZ_Offset.data_ptr(), 0, NZ.numel(),
         K_Global, out.data_ptr(), 8 * M_Global, 8, M_Global, ws.data_ptr(), ws.numel(), 0, 0, st.data_ptr(), _stream())
@@ -215,7 +226,7 @@ def decode_attention(q: torch.Tensor, k_store: SparseStore, v_store: SparseStore
         Lmax = min(k_store.max_tokens, v_store.max_tokens)
         _, nbytes = plan(n_kv, Lmax, W, group, nsplit)
         ws = _take_workspace(workspace, q.device, nbytes)
-        r = _lib.lib().mfar_decode_attention_fp16_dyn(
+        r = _lib.native().mfar_decode_attention_fp16_dyn(
             q.data_ptr(), q.stride(0), n_kv, group,
             k_store.bitmaps.data_ptr(), k_store.tiles_cap, k_store.accum.data_ptr(), k_store.tiles_cap + 1,
             k_store.nz.data_ptr(), None, k_store.nz_capacity, k_store.nz.numel(),
@@ -229,7 +240,7 @@ def decode_attention(q: torch.Tensor, k_store: SparseStore, v_store: SparseStore
         return out
     _, nbytes = plan(n_kv, L, W, group, nsplit)
     ws = _take_workspace(workspace, q.device, nbytes)
-    r = _lib.lib().mfar_decode_attention_fp16(
+    r = _lib.native().mfar_decode_attention_fp16(
         q.data_ptr(), q.stride(0), n_kv, group,
         k_store.bitmaps.data_ptr(), k_store.tiles_cap, k_store.accum.data_ptr(), k_store.tiles_cap + 1,
         k_store.nz.data_ptr(), None, k_store.nz_capacity, k_store.nz.numel(),

@@ -59,7 +59,7 @@ def mustafar_key_formulation_quant(bmp, NZ_quant, tile_offsets, scales, zeros, B
     out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
     st = _dev_status(B.device)
     rows = B.shape[1] if B.dim() == 3 else 1
-    r = _lib.lib().mfar_key_scores_rows_quant(
+    r = _lib.native().mfar_key_scores_rows_quant(
         B.data_ptr(), rows * K_Global, n_kv, num_key_value_groups, bmp.data_ptr(), tiles, tile_offsets.data_ptr(),
         scales.data_ptr(), zeros.data_ptr(), tiles, NZ_quant.data_ptr(), NZ_quant.numel(), M_Global, bit,
         _qgroup(scales, n_kv, tiles), out.data_ptr(), 8 * M_Global, 8, M_Global, st.data_ptr(), _stream())
@@ -87,7 +87,7 @@ def _value(bmp, NZ_quant, tile_offsets, scales, zeros, P, probs_stride, M_Global
     _, nbytes = plan(n_kv, K_Global, 0, groups)
     ws = _workspace(P.device, max(nbytes, 65536 + n_kv * max(1, K_Global // 64) * groups * 132 * 4))
     st = _dev_status(P.device)
-    r = _lib.lib().mfar_value_output_rows_quant(
+    r = _lib.native().mfar_value_output_rows_quant(
         P.data_ptr(), probs_stride, n_kv, groups, bmp.data_ptr(), tiles, tile_offsets.data_ptr(), scales.data_ptr(),
         zeros.data_ptr(), tiles, NZ_quant.data_ptr(), NZ_quant.numel(), K_Global, bit, _qgroup(scales, n_kv, tiles),
         out.data_ptr(), out_stride, out_stride // M_Global, M_Global, ws.data_ptr(), ws.numel(), 0, st.data_ptr(), _stream())
@@ -163,7 +163,7 @@ def decode_attention_quant(q, kq: dict, vq: dict, n_tokens: int, k_window, v_win
     if int(vq.get("head_stride", tiles)) != hs:
         raise RuntimeError("key and value tensors must share their head stride")
     qg = _qgroup(kq["scales"], n_kv, hs) if n_tokens else 64
-    r = _lib.lib().mfar_decode_attention_quant(
+    r = _lib.native().mfar_decode_attention_quant(
         q.data_ptr(), q.stride(0), n_kv, group,
         kq["bitmaps"].data_ptr(), kq["tile_offsets"].data_ptr(), kq["scales"].data_ptr(), kq["zeros"].data_ptr(),
         kq["packed"].data_ptr(), kq["packed"].numel(),

@@ -7,12 +7,10 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from .compression import _stream
+from .ops import _dev_status
 
 D = 128
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _need(t: torch.Tensor, what: str):
@@ -34,7 +32,7 @@ def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tenso
         raise RuntimeError("add_rmsnorm: weight does not match the hidden size")
     if out is None:
         out = torch.empty_like(x)
-    _lib.check(_lib.lib().mfar_add_rmsnorm_f16(x.data_ptr(), None if delta is None else delta.data_ptr(), weight.data_ptr(),
+    _lib.check(_lib.native().mfar_add_rmsnorm_f16(x.data_ptr(), None if delta is None else delta.data_ptr(), weight.data_ptr(),
                                                out.data_ptr(), x.numel() // hidden, hidden, float(eps), _stream()),
                "mfar_add_rmsnorm_f16")
     return out
@@ -77,12 +75,11 @@ def rope_append(qkv: torch.Tensor, inv_freq: torch.Tensor, pos, slot, n_q_heads:
         if int(v) < 0:
             raise RuntimeError(f"rope_append: negative {name}")
         return None, int(v)
-    from .ops import _dev_status
     pd, ph = dev_or_host(pos, "pos")
     sd, sh = dev_or_host(slot, "slot")
     if sd is None and sh >= k_window.shape[1]:
         raise RuntimeError("rope_append: slot beyond the window capacity")
-    _lib.check(_lib.lib().mfar_rope_append_f16(qkv.data_ptr(), inv_freq.data_ptr(), pd, ph, sd, sh, B, n_q_heads, n_kv_heads,
+    _lib.check(_lib.native().mfar_rope_append_f16(qkv.data_ptr(), inv_freq.data_ptr(), pd, ph, sd, sh, B, n_q_heads, n_kv_heads,
                                                q_out.data_ptr(), k_window.data_ptr(), v_window.data_ptr(),
                                                k_window.stride(0), k_window.stride(1), k_window.shape[1],
                                                int(prune_rank), int(prune_back),
@@ -98,5 +95,5 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Te
     rows = gate_up.numel() // (2 * width)
     if out is None:
         out = torch.empty(gate_up.shape[:-1] + (width,), dtype=torch.float16, device=gate_up.device)
-    _lib.check(_lib.lib().mfar_silu_mul_f16(gate_up.data_ptr(), out.data_ptr(), rows, width, _stream()), "mfar_silu_mul_f16")
+    _lib.check(_lib.native().mfar_silu_mul_f16(gate_up.data_ptr(), out.data_ptr(), rows, width, _stream()), "mfar_silu_mul_f16")
     return out
