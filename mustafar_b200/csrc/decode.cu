@@ -355,6 +355,7 @@ static int block_split(int n_kv_heads, int nblk, int hint) {
     int ns = hint > 0 ? hint : model_split_count(n_kv_heads, nblk, min_ns, 128, device_sm_count());
     if (ns < min_ns) ns = min_ns;
     if (ns > nblk) ns = nblk;
+    if (ns > kMaxSplits && min_ns <= kMaxSplits) ns = kMaxSplits;   // the merge's weights live in shared memory
     if (ns < 1) ns = 1;
     const int bps = (nblk + ns - 1) / ns;
     return (nblk + bps - 1) / bps;   // no empty splits
@@ -368,7 +369,7 @@ extern "C" int mfar_decode_plan(int n_kv_heads, int n_tokens, int window, int ns
     if (nsplit_out) *nsplit_out = ns;
     if (workspace_bytes)
         *workspace_bytes = counters_bytes(n_kv_heads) +
-                           static_cast<size_t>(n_kv_heads) * (ns + 1) * group * kPartialStride * sizeof(float) + 16;
+                           static_cast<size_t>(n_kv_heads) * (ns + window_records(window)) * group * kPartialStride * sizeof(float) + 16;
     return MFAR_OK;
 }
 
@@ -401,7 +402,10 @@ static int decode_attention_fp16_impl(
     size_t need = 0;
     int r = mfar_decode_plan(n_kv_heads, n_tokens, window, nsplit, &ns, &need, group);
     if (r) return r;
-    if (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)) return MFAR_ERR_WORKSPACE;
+    // room for one window record is enough: fewer CTAs then share the window
+    const size_t record = static_cast<size_t>(n_kv_heads) * group * kPartialStride * sizeof(float);
+    if (workspace_bytes < counters_bytes(n_kv_heads) + (ns + 1) * record || (reinterpret_cast<uintptr_t>(workspace) & 15))
+        return MFAR_ERR_WORKSPACE;
 
     DecodeParams p{};
     p.k = Sparse{reinterpret_cast<const unsigned long long*>(k_bitmaps), k_accum, static_cast<const __half*>(k_nz),
@@ -428,7 +432,7 @@ static int decode_attention_fp16_impl(
     p.dev_status = dev_status;
     p.nsplit = ns;
     p.bps = ns > 0 ? (p.nblk + ns - 1) / ns : 0;
-    p.nrec = ns + (window > 0 ? 1 : 0);
+    split_window(p, n_kv_heads, device_sm_count(), static_cast<long long>((workspace_bytes - counters_bytes(n_kv_heads)) / record));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     r = launch_decode_attn(p, group, n_kv_heads, p.nrec, s);
     if (r || p.counters) return r;

@@ -1,6 +1,6 @@
 // Fused decode attention over the bitmap + packed-fp16 cache:
 //   q.K^T over the compressed tokens, online softmax, P.V, split-KV partial records, and the merge of the
-//   records by the CTA that finishes a kv head last (one launch per call); one extra CTA per kv head handles
+//   records by the CTA that finishes a kv head last (one launch per call); further CTAs per kv head handle
 //   the dense recent-token window.
 //
 // A CTA (4 warps) walks a range of 64-token blocks of ONE kv head and serves all G query heads that share it, so
@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tb = lane >> 2, cp = lane & 3;   // fragment row (= bitmap byte) and k pair of this lane
     const int h = blockIdx.y;
-    const int split = blockIdx.x + p.split_offset;
-    const bool is_window = split == p.nsplit;
+    const int split = blockIdx.x;
+    const bool is_window = split >= p.nsplit;
     unsigned sel, mh, ml;
     lane_byte_constants(tb, sel, mh, ml);
 
@@ -342,9 +342,9 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
         nblk = max(0, min(*p.L_dev / 64, p.nblk));
         bps = p.nsplit > 0 ? (nblk + p.nsplit - 1) / p.nsplit : 0;
     }
-    const int blk0 = is_window ? 0 : split * bps;
+    const int blk0 = is_window ? (split - p.nsplit) * p.wbps : split * bps;
     const int W = (is_window && p.W_dev) ? max(0, min(*p.W_dev, p.W)) : p.W;
-    int nb = is_window ? (W + 63) / 64 : min(bps, nblk - blk0);
+    int nb = is_window ? min(p.wbps, (W + 63) / 64 - blk0) : min(bps, nblk - blk0);
     if (nb < 0) nb = 0;
 
     // ---- prologue
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
                 const int c = warp * 32 + kg * 16 + 2 * cp;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int t0 = i * 64 + 8 * tb + j, t1 = t0 + 4;
+                    const int t0 = (blk0 + i) * 64 + 8 * tb + j, t1 = t0 + 4;
                     unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0;
                     if (t0 < W) { a0 = ldg_nc_u32(kw + t0 * p.win_ts + c); a2 = ldg_nc_u32(kw + t0 * p.win_ts + c + 8); }
                     if (t1 < W) { a1 = ldg_nc_u32(kw + t1 * p.win_ts + c); a3 = ldg_nc_u32(kw + t1 * p.win_ts + c + 8); }
@@ -607,8 +607,8 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
                 s0 *= p.scale_log2;
                 s1 *= p.scale_log2;
                 if (is_window) {
-                    if (i * 64 + tok0 >= W) s0 = -INFINITY;
-                    if (i * 64 + tok1 >= W) s1 = -INFINITY;
+                    if ((blk0 + i) * 64 + tok0 >= W) s0 = -INFINITY;
+                    if ((blk0 + i) * 64 + tok1 >= W) s1 = -INFINITY;
                 }
                 const float m_new = fmaxf(m_run[j], warp_max_f32(fmaxf(s0, s1)));
                 const float a = fast_exp2(m_run[j] - m_new);   // exp2(-inf) = 0 on the first block
@@ -671,8 +671,8 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
                             r[2] = __byte_perm(x.y, x.w, 0x5410); r[3] = __byte_perm(x.y, x.w, 0x7632);
                         }
                     };
-                    row(i * 64 + t, r1);
-                    row(i * 64 + t + 1, r2);
+                    row((blk0 + i) * 64 + t, r1);
+                    row((blk0 + i) * 64 + t + 1, r2);
                 }
                 mma_step<G>(dv[hf], r1, r2, bf, pp);
             }
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
     // warp w merges heads w, w + 4: its lanes fetch the records' (m, l) in parallel, the weights go through shared
     // memory (the reduction buffer is free again), then every lane sums four channels over the records
     const int nrec = p.nrec;
-    float* wgt = red;   // [G][nrec], nrec <= 129
+    float* wgt = red;   // [G][nrec], nrec <= kMaxSplits + kMaxWindowSplits < 4 * kD
     for (int g = warp; g < G; g += kAWarps) {
         const float* base = record_ptr(p, G, h, 0, g);
         const int64_t step = static_cast<int64_t>(G) * kPartialStride;

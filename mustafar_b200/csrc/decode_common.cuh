@@ -172,6 +172,7 @@ constexpr int kPartL = kD + 1;
 enum { MODE_KEY = 1, MODE_VALUE = 2 };
 constexpr int kSlackHalves = 64;  // a decode never reads further than this past a stage's values
 constexpr int kMaxBlocksPerSplit = 256;
+constexpr int kMaxSplits = 480;    // per kv head, whatever a caller asks for
 
 struct Sparse {
     const unsigned long long* bmp;
@@ -225,7 +226,7 @@ struct DecodeParams {
     const __half* p_in;    // MODE_VALUE: [Bq][p_stride]
     int64_t p_stride;
     unsigned* dev_status;
-    int split_offset;      // added to blockIdx.x (lets a launch cover only the window record)
+    int nwin, wbps;        // CTAs (and records) per kv head for the dense window behind the nsplit ones, 64-token blocks each
     // fused attention only: the CTA that finishes a kv head last merges its records into out
     unsigned* counters;    // one per kv head, zero between launches; NULL = no merge (a combine launch follows)
     __half* out;
@@ -270,6 +271,35 @@ __device__ __forceinline__ void zero_score_rows(__half* block, int64_t head_stri
         *reinterpret_cast<uint4*>(block + g * head_stride + r * row_stride + 8 * (i & 7)) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
+// The dense window of a kv head is dealt out over p.nwin CTAs of p.wbps 64-token blocks.  A window block reads its K and
+// then its V rows straight from global memory, two exposed trips per block, so a CTA with the 5 blocks of 300 tokens
+// outlasts a whole short split.  While the grid stays under 4 CTAs per SM every block gets its own CTA; beyond that a
+// window CTA takes as many blocks as half a split, which saves prologues and records.  One CTA for the whole
+// window against this: 64 sequences x 32768 tokens, window 128, 1327 -> 1311 us; the attention of a step over 4 x 2048 tokens,
+// window 201 of 384, 4 us less; no shape measured slower.  records: what the workspace has room
+// for (at least nsplit + 1).
+constexpr int kMaxWindowSplits = 16;
+inline int window_records(int window) {
+    const int nwb = (window + 63) / 64;
+    return nwb < 1 ? 1 : (nwb < kMaxWindowSplits ? nwb : kMaxWindowSplits);
+}
+inline void split_window(DecodeParams& p, int n_kv_heads, int n_sm, long long records) {
+    const int nwb = (p.W + 63) / 64;
+    p.nwin = p.wbps = 0;
+    if (nwb > 0) {
+        const bool roomy = static_cast<long long>(n_kv_heads) * (p.nsplit + nwb) <= 4ll * n_sm;
+        int wb = roomy ? 1 : (p.bps / 2 < 1 ? 1 : p.bps / 2);
+        long long most = records - p.nsplit;
+        if (most > kMaxWindowSplits) most = kMaxWindowSplits;
+        const int least = static_cast<int>((nwb + most - 1) / most);
+        if (wb < least) wb = least;
+        if (wb > nwb) wb = nwb;
+        p.wbps = wb;
+        p.nwin = (nwb + wb - 1) / wb;
+    }
+    p.nrec = p.nsplit + p.nwin;
+}
+
 // Split count of the 64-token-block decode kernels.  The grid is n_kv_heads * ns CTAs of bps = ceil(nblk / ns) blocks.
 // The cost of a candidate follows a model fitted to a measured sweep of ns over batch 1..64 and
 // 4k..32k tokens on a B200 (all times in units of one block on an otherwise idle SM, ~2 us):

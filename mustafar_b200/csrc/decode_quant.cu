@@ -352,6 +352,7 @@ static void q_split(int n_kv_heads, int nblk, int hint, int* ns, int* bps) {
     const int max_n = (nblk + 1) / 2;   // what callers size their workspace for
     int n = hint > 0 ? hint : model_split_count(n_kv_heads, nblk, 1, max_n < 128 ? max_n : 128, device_sm_count());
     if (n > nblk) n = nblk;
+    if (n > kMaxSplits) n = kMaxSplits;   // the merge's weights live in shared memory
     if (n < 1) n = 1;
     *bps = (nblk + n - 1) / n;
     *ns = (nblk + *bps - 1) / *bps;
@@ -474,9 +475,11 @@ extern "C" int mfar_decode_attention_quant(
         p.nblk = n_tokens / 64;
         q_split(n_kv_heads, p.nblk, nsplit, &p.nsplit, &p.bps);
     }
-    p.nrec = p.nsplit + (window > 0 ? 1 : 0);
-    const size_t need = counters_bytes(n_kv_heads) + static_cast<size_t>(n_kv_heads) * p.nrec * group * kPartialStride * sizeof(float);
+    const size_t record = static_cast<size_t>(n_kv_heads) * group * kPartialStride * sizeof(float);
+    const size_t need = counters_bytes(n_kv_heads) + (p.nsplit + (window > 0 ? 1 : 0)) * record;
     if (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)) return MFAR_ERR_WORKSPACE;
+    p.W = window;
+    split_window(p, n_kv_heads, device_sm_count(), static_cast<long long>((workspace_bytes - counters_bytes(n_kv_heads)) / record));
     p.kq = QSparse{reinterpret_cast<const unsigned long long*>(k_bitmaps), k_tile_offsets,
                    static_cast<const __half*>(k_scales), static_cast<const __half*>(k_zeros),
                    reinterpret_cast<const unsigned*>(k_packed), bmp_head_stride, meta_head_stride, k_packed_words};
@@ -489,7 +492,6 @@ extern "C" int mfar_decode_attention_quant(
     p.vwin = static_cast<const __half*>(v_window);
     p.win_hs = win_head_stride;
     p.win_ts = win_token_stride;
-    p.W = window;
     p.W_dev = window_len_dev;
     p.L_dev = n_tokens_dev;
     p.cap = 8;

@@ -224,7 +224,8 @@ def decode_attention(q: torch.Tensor, k_store: SparseStore, v_store: SparseStore
         if stage_halves is None:
             raise RuntimeError("n_tokens on the device needs an explicit stage_halves bound")
         Lmax = min(k_store.max_tokens, v_store.max_tokens)
-        _, nbytes = plan(n_kv, Lmax, W, group, nsplit)
+        # a caller's workspace may be the smallest one (the window in one record); the default one has room for all
+        _, nbytes = plan(n_kv, Lmax, W if workspace is None else 0, group, nsplit)
         ws = _take_workspace(workspace, q.device, nbytes)
         r = _lib.native().mfar_decode_attention_fp16_dyn(
             q.data_ptr(), q.stride(0), n_kv, group,
@@ -238,7 +239,7 @@ def decode_attention(q: torch.Tensor, k_store: SparseStore, v_store: SparseStore
         if _debug_check():
             check_device_status(q.device)
         return out
-    _, nbytes = plan(n_kv, L, W, group, nsplit)
+    _, nbytes = plan(n_kv, L, W if workspace is None else 0, group, nsplit)
     ws = _take_workspace(workspace, q.device, nbytes)
     r = _lib.native().mfar_decode_attention_fp16(
         q.data_ptr(), q.stride(0), n_kv, group,

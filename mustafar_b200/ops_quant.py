@@ -153,7 +153,9 @@ def decode_attention_quant(q, kq: dict, vq: dict, n_tokens: int, k_window, v_win
         softmax_scale = 1.0 / math.sqrt(D)
     if out is None:
         out = torch.empty((n_kv * group, D), dtype=torch.float16, device=q.device)
-    ws = _take_workspace(workspace, q.device, 65536 + n_kv * (max(1, n_tokens // 64) + 1) * group * 132 * 4)
+    # (the default workspace has room for all the records a window may be split into)
+    records = max(1, n_tokens // 64) + (16 if workspace is None else 1)
+    ws = _take_workspace(workspace, q.device, 65536 + n_kv * records * group * 132 * 4)
     for t, name in ((n_tokens_dev, "n_tokens_dev"), (window_len, "window_len")):
         if t is not None and (not t.is_cuda or t.dtype != torch.int32 or t.numel() != 1):
             raise RuntimeError(f"{name} must be a CUDA int32 tensor with one element")

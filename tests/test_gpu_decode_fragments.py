@@ -72,3 +72,42 @@ def test_fp16_tiles(G, L):
     assert oracle.rel_l2(o[:, 0].cpu(), oracle.value_formulation_ref(v, pr, G)) < TOL
     assert not o[:, 1:].any()
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("heads,L", [(2, 0), (2, 192), (300, 64)])          # window CTAs of one block, and of several
+@pytest.mark.parametrize("W", [1, 63, 64, 65, 129, 300, 1100])
+@pytest.mark.parametrize("bits", [16, 2])
+def test_window_split(heads, L, W, bits):
+    from mustafar_b200 import compression as c, compression_quant as cq, ops, ops_quant
+    G = 4
+    k, v = oracle.make_kv(heads, max(L, 64) + W, seed=8)
+    q = oracle.make_query(heads * G, seed=9)
+    kc, vc, kw, vw = k[:, :L].contiguous(), v[:, :L].contiguous(), k[:, max(L, 64):].contiguous(), v[:, max(L, 64):].contiguous()
+    capacity = W + 70                       # a window buffer longer than the valid part, its length on the device
+    kb, vb = (torch.full((heads, capacity, 128), float("nan"), dtype=torch.float16) for _ in range(2))
+    kb[:, :W], vb[:, :W] = kw, vw
+    wl = torch.tensor([W], dtype=torch.int32, device="cuda")
+    sample = [0, heads // 2, heads - 1]
+    rows = [h * G + g for h in sample for g in range(G)]
+    if bits == 16:
+        ks, vs = (c.SparseStore(heads, max(L, 64), kind, "cuda") for kind in (c.KEY, c.VALUE))
+        if L:
+            ks.append(kc.cuda()), vs.append(vc.cuda())
+        least = ops.plan(heads, L, 0, G)[1]
+        small = ops.new_workspace(torch.device("cuda", 0), least)[:least]
+        got = [ops.decode_attention(q.cuda(), ks, vs, kw.cuda(), vw.cuda(), G),
+               ops.decode_attention(q.cuda(), ks, vs, kb.cuda(), vb.cuda(), G, window_len=wl),
+               ops.decode_attention(q.cuda(), ks, vs, kw.cuda(), vw.cuda(), G, workspace=small)]
+        want = oracle.decode_attention_ref(q[rows], kc[sample], vc[sample], kw[sample], vw[sample], G)
+    else:
+        if not L:
+            pytest.skip("covered with the fp16 cache")
+        kq, vq = cq.compress_quant(kc.cuda(), c.KEY), cq.compress_quant(vc.cuda(), c.VALUE)
+        kd = oracle.dequant_key_ref(oracle.quant_compress_key_ref(kc[sample]), L)
+        vd = oracle.dequant_value_ref(oracle.quant_compress_value_ref(vc[sample]), L)
+        got = [ops_quant.decode_attention_quant(q.cuda(), kq, vq, L, kw.cuda(), vw.cuda(), G),
+               ops_quant.decode_attention_quant(q.cuda(), kq, vq, L, kb.cuda(), vb.cuda(), G, window_len=wl)]
+        want = oracle.decode_attention_ref(q[rows], kd, vd, kw[sample], vw[sample], G)
+    ops.check_device_status()
+    for out in got:
+        assert oracle.rel_l2(out[rows].float().cpu(), want) < TOL
