@@ -13,6 +13,9 @@
 //      code into the tile's word: 32/bits codes per uint32, least significant first.
 // bits = 2, group = 64 reproduces kernel_quant/compression_quant.py bit for bit; bits = 4 and
 // group = 32 (a fresh scale / zero every 32 nonzeros of a tile) extend it.
+// Bits and group are compile-time (a code's word and shift cost no division), a run of codes is collected in a register
+// and or-ed once per word, and a tile's range is taken while its values are packed: K and V of 4 x 4928 tokens, 2 bits,
+// 142 -> 133 us.  Bound by latency and issue (K: 53 % of the issue slots, V: 71 %).
 #include "compress_common.cuh"
 
 namespace mfar {
