@@ -12,7 +12,7 @@
 // probabilities it reads from the caller's array as the B operand; split partials are summed by combine_kernel.
 // Against fp32 multiply-adds per position and head: the pair of products over 8 sequences x 16384 tokens with 4 query
 // heads per kv head 177 -> 147 us (the zero fill of the padded scores included).
-#include "decode_common.cuh"
+#include "decode_plain.cuh"
 
 namespace mfar {
 
@@ -41,7 +41,7 @@ struct SmemLayout {
 };
 
 template <int G, int MODE>
-__global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
+__global__ void __launch_bounds__(kThreads, 5) spmv_kernel(const __grid_constant__ DecodeParams p) {
     static_assert(MODE == MODE_KEY || MODE == MODE_VALUE, "single-product kernel");
     extern __shared__ __align__(128) unsigned char smem[];
     const SmemLayout<G, MODE> lay(p.cap);
@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
 
     bool timed_out = false;
     int done = 0;   // blocks finished
+    bool has_nan = false;
     for (int i = 0; i < nb; ++i) {
         const unsigned char* st = smem + lay.stages + static_cast<size_t>(i % kStages) * stg;
         const uint2* bm_s = reinterpret_cast<const uint2*>(st);
@@ -192,6 +193,7 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
                 }
                 *reinterpret_cast<__half2*>(p.s_out + (static_cast<int64_t>(h) * G + g) * p.s_stride +
                                             static_cast<int64_t>(blk0 + i) * 64 + 2 * lane) = __floats2half2_rn(s0, s1);
+                has_nan |= s0 != s0 || s1 != s1;
             }
         } else {
 #pragma unroll
@@ -215,7 +217,11 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
         }
         return;
     }
-    if (MODE == MODE_KEY) return;
+    // a NaN may be the partner's infinity or a zero's product with one: once more without pairs
+    if (MODE == MODE_KEY) {
+        if (__syncthreads_or(has_nan)) plain_key_scores<G>(p, h, blk0, nb, red);
+        return;
+    }
 
     // ---- VALUE epilogue: sum the 4 warps and write the partial
     __syncthreads();
@@ -238,7 +244,9 @@ __global__ void __launch_bounds__(kThreads, 5) spmv_kernel(DecodeParams p) {
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) s += red[(static_cast<size_t>(w) * G + g) * kD + c];
         rec[g * kPartialStride + c] = s;
+        has_nan |= s != s;
     }
+    if (__syncthreads_or(has_nan)) plain_value_record<G>(p, h, split, blk0, nb);
 }
 
 // Merges the split partials of one q head: out = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M)

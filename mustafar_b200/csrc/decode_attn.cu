@@ -29,7 +29,7 @@
 // and one rounded product, which gives the same bits (zero-points outside +-1024 go through fp32).  Against one
 // predicated step per position: 32 x 16384 tokens of 2-bit codes 583 -> 450 us, 8 x 4096 of 4-bit codes with a scale per
 // 32 nonzeros, half of the values kept, 82.7 -> 69.6 us.  Bound by the integer pipe and issue (both about 60 %).
-#include "decode_common.cuh"
+#include "decode_plain.cuh"
 
 namespace mfar {
 
@@ -310,7 +310,7 @@ __device__ __forceinline__ float* record_ptr(const DecodeParams& p, int G, int h
 
 // 5 CTAs per SM (96 registers); the quantised cache with 8 heads needs two accumulator sets and would spill at 96
 template <int G, int QBITS, bool GROUP32>
-__global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) decode_attn_kernel(DecodeParams p) {
+__global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) decode_attn_kernel(const __grid_constant__ DecodeParams p) {
     constexpr bool QUANT = QBITS != 0;
     using QB = AttnQBuf<QUANT ? QBITS : 2, GROUP32>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -697,12 +697,14 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
                     if (g < G) red[(static_cast<size_t>(warp) * G + g) * kD + hf * 64 + 8 * tb + c] = dv[hf][f][j][e];
                 }
     __syncthreads();
+    bool has_nan = false;
     for (int idx = tid; idx < G * kD; idx += kAThreads) {
         const int g = idx / kD, c = idx % kD;
         float s = 0.f;
 #pragma unroll
         for (int w = 0; w < kAWarps; ++w) s += red[(static_cast<size_t>(w) * G + g) * kD + c];
         record_ptr(p, G, h, split, g)[c] = timed_out ? 0.f : s;
+        has_nan |= s != s;
     }
 #pragma unroll
     for (int j = 0; j < kHeadsPerWarp; ++j) {
@@ -719,9 +721,14 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
 
     // ---- merge: the CTA that arrives last at this kv head's counter combines all records
     //      out = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M)
-    if (p.counters == nullptr) return;
     __threadfence();
-    __syncthreads();
+    // an infinity or NaN has reached its partner's row, too (a NaN probability reaches every channel): once more without pairs
+    if (__syncthreads_or(has_nan && !timed_out)) {
+        plain_attention<G, QBITS, GROUP32>(p, h, split, blk0, nb, W, red, ps, kPsStride, alpha_s);
+        __threadfence();
+        __syncthreads();
+    }
+    if (p.counters == nullptr) return;
     if (tid == 0) {
         const unsigned arrived = atomicAdd(p.counters + h, 1u) + 1u;
         s_last = arrived == gridDim.x;

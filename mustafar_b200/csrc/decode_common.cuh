@@ -112,7 +112,8 @@ __device__ __forceinline__ void expand_tile(unsigned lo, unsigned hi, const unsi
 
 // Where a tile's coefficient (query channel, probability) goes in the B operand: a register of A holds two positions of
 // ONE tile, so it enters B as (c, 0) for the first position and as (0, c) for the second.  Up to 4 query heads fill the 8
-// columns with both forms (column = head + 4 * form); 8 heads take one mma per form.
+// columns with both forms (column = head + 4 * form); 8 heads take one mma per form.  The zero does not take an infinity or a
+// NaN away: results with a NaN are computed again without pairs (decode_plain.cuh).
 template <int G>
 struct BForms {
     static constexpr int FORMS = G == 8 ? 2 : 1;
