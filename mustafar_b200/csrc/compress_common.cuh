@@ -194,23 +194,25 @@ __device__ __forceinline__ long long lookback_exclusive(unsigned long long* st, 
 // Chains of at most kClusterBlocks blocks (a decode append is 4) run as one thread-block cluster per head: the blocks
 // hand their totals to each other through distributed shared memory, so there is no ticket, no status word to poll and no
 // scratch to clear beforehand.  cluster_open .. cluster_announce .. cluster_exclusive, called by all threads of the CTA in
-// this order; work in between hides the two cluster barriers.
+// this order; work in between hides the two cluster barriers.  The barriers are the forms without .aligned: they come after
+// divergent code, and .aligned would need every warp to arrive as one.  They have no time limit: every CTA of a cluster is
+// resident, and none leaves its kernel between the two arrivals.
 constexpr int kClusterBlocks = 8;   // the portable cluster size
 
-__device__ __forceinline__ void cluster_open() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_open() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 // totals[b] of every CTA of the cluster (nblk of them) receives this block's total; thread r writes to CTA r
 __device__ __forceinline__ void cluster_announce(unsigned* totals, int b, int nblk, unsigned total) {
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA has started: its shared memory exists
+    asm volatile("barrier.cluster.wait;" ::: "memory");   // every CTA has started: its shared memory exists
     if (static_cast<int>(threadIdx.x) < nblk) {
         unsigned remote;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(totals + b)), "r"(threadIdx.x));
         asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(total) : "memory");
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
 }
 // sum of the totals before block b; nobody writes to this CTA any more when it returns
 __device__ __forceinline__ unsigned cluster_exclusive(const unsigned* totals, int b) {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     unsigned excl = 0;
     for (int i = 0; i < b; ++i) excl += totals[i];
     return excl;
