@@ -6,10 +6,10 @@ namespace mfar {
 int device_sm_count() {
     static int cached[64] = {0};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return 148;
     if (cached[dev] == 0) {
         int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        if (!cuda_ok(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) || n <= 0) n = 148;
         cached[dev] = n;
     }
     return cached[dev];

@@ -57,6 +57,13 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) {
 // multiprocessors of the current device (queried once per device; api_misc.cu)
 int device_sm_count();
 
+// a failed call's error stays for the next cudaGetLastError: whoever reports it takes it off, or a later launch that went
+// well is reported in its place
+inline bool cuda_ok(cudaError_t e) {
+    if (e == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? MFAR_OK : MFAR_ERR_LAUNCH; }
 
 }  // namespace mfar

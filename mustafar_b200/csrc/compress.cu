@@ -336,7 +336,7 @@ extern "C" int mfar_compress_fp16(const void* x, int64_t x_head_stride, int64_t 
     // a cluster per head up to the portable cluster size: 256 heads x 256 tokens of K and of V
     // take 33.3 us against 39.0 us with the look-back (a memset, tickets and polls less)
     const bool cluster = nblk <= kClusterBlocks;
-    if (!cluster && cudaMemsetAsync(scratch, 0, need, s) != cudaSuccess) return MFAR_ERR_LAUNCH;
+    if (!cluster && !cuda_ok(cudaMemsetAsync(scratch, 0, need, s))) return MFAR_ERR_LAUNCH;
 
     CompressParams p;
     p.x = static_cast<const __half*>(x);
@@ -421,10 +421,10 @@ extern "C" int mfar_compress_fp16_noalloc(const void* x, int64_t x_head_stride, 
     if (n_heads < 0 || n_tokens < 0 || (n_tokens % 64) != 0) return MFAR_ERR_ARG;
     if (static_cast<int64_t>(n_heads) * (n_tokens / 64) > MFAR_NOALLOC_MAX_BLOCKS) return MFAR_ERR_LIMIT;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
     if (g_static_scratch_addr[dev] == nullptr) {
         void* addr = nullptr;
-        if (cudaGetSymbolAddress(&addr, g_static_scratch) != cudaSuccess || addr == nullptr) return MFAR_ERR_LAUNCH;
+        if (!cuda_ok(cudaGetSymbolAddress(&addr, g_static_scratch)) || addr == nullptr) return MFAR_ERR_LAUNCH;
         g_static_scratch_addr[dev] = addr;
     }
     return mfar_compress_fp16(x, x_head_stride, x_token_stride, 0, 0, n_heads, n_tokens, kind, prune_rank, bitmaps,

@@ -231,7 +231,7 @@ inline int launch_clusters(void (*kernel)(Params), const Params& p, unsigned gri
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? MFAR_OK : MFAR_ERR_LAUNCH;
+    return cuda_ok(cudaLaunchKernelEx(&cfg, kernel, p)) ? MFAR_OK : MFAR_ERR_LAUNCH;
 }
 
 }  // namespace mfar

@@ -408,7 +408,7 @@ extern "C" int mfar_compress_quant(const void* x, int64_t x_head_stride, int64_t
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // a cluster per head up to the portable cluster size (one chain over all heads stays with the look-back)
     const bool cluster = nblk <= kClusterBlocks && (packed_head_stride > 0 || n_heads == 1);
-    if (!cluster && cudaMemsetAsync(scratch, 0, need, s) != cudaSuccess) return MFAR_ERR_LAUNCH;
+    if (!cluster && !cuda_ok(cudaMemsetAsync(scratch, 0, need, s))) return MFAR_ERR_LAUNCH;
 
     QuantParams p;
     p.x = static_cast<const __half*>(x);

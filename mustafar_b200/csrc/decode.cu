@@ -310,10 +310,10 @@ static int launch_spmv(const DecodeParams& p, int n_kv_heads, int grid_x, cudaSt
     const SmemLayout<G, MODE> lay(p.cap);
     static size_t configured[64] = {0};   // largest dynamic shared memory size opted into so far, per device
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
     if (lay.total > configured[dev]) {
-        if (cudaFuncSetAttribute(spmv_kernel<G, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(lay.total)) != cudaSuccess)
+        if (!cuda_ok(cudaFuncSetAttribute(spmv_kernel<G, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(lay.total))))
             return MFAR_ERR_LAUNCH;
         configured[dev] = lay.total;
     }

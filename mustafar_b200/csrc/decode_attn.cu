@@ -788,10 +788,10 @@ static int launch_attn(const DecodeParams& p, int n_kv_heads, int grid_x, cudaSt
     const AttnLayout lay(p.cap, G, QBITS ? sizeof(AttnQBuf<QBITS ? QBITS : 2, GROUP32>) : 0);
     static size_t configured[64] = {0};   // largest dynamic shared memory size opted into so far, per device
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
     if (lay.total > configured[dev]) {
-        if (cudaFuncSetAttribute(decode_attn_kernel<G, QBITS, GROUP32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(lay.total)) != cudaSuccess)
+        if (!cuda_ok(cudaFuncSetAttribute(decode_attn_kernel<G, QBITS, GROUP32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(lay.total))))
             return MFAR_ERR_LAUNCH;
         configured[dev] = lay.total;
     }

@@ -304,10 +304,10 @@ static int launch_q(const QDecodeParams& p, int n_kv_heads, cudaStream_t s) {
     const QLayout<G, MODE, BITS> lay;
     static bool configured[64] = {false};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return MFAR_ERR_LAUNCH;
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(decode_quant_kernel<G, MODE, BITS, GROUP32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(lay.total)) != cudaSuccess)
+        if (!cuda_ok(cudaFuncSetAttribute(decode_quant_kernel<G, MODE, BITS, GROUP32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(lay.total))))
             return MFAR_ERR_LAUNCH;
         configured[dev] = true;
     }
