@@ -18,6 +18,11 @@ import torch
 from . import _lib
 from .compression import D, SparseStore, _stream
 
+# The fused kernels deal a window out over at most 16 records of 64 tokens or more.  The default workspace always has room
+# for them: its size then depends on the heads and the compressed length alone, so that a call with a short window warms up
+# the capture of one with a long window, and no longer window moves a buffer that a captured graph writes to.
+WINDOW_ROOM = 16 * 64
+
 _workspaces: dict = {}
 _status: dict = {}
 
@@ -158,7 +163,7 @@ def mustafar_value_formulation(bmp, NZ, idx, NZ_Offset, B, Reduction_Workspace, 
     n_kv = Batch_Size // num_key_value_groups
     tiles = M_Global * K_Global // 64
     out = torch.empty((Batch_Size, 8, M_Global), dtype=torch.float16, device=B.device)
-    _, nbytes = plan(n_kv, K_Global, 0, num_key_value_groups)
+    _, nbytes = plan(n_kv, K_Global, WINDOW_ROOM, num_key_value_groups)
     ws = _workspace(B.device, nbytes)
     st = _dev_status(B.device)
     rows = Bc.shape[1] if Bc.dim() == 3 else 1
@@ -224,8 +229,8 @@ def decode_attention(q: torch.Tensor, k_store: SparseStore, v_store: SparseStore
         if stage_halves is None:
             raise RuntimeError("n_tokens on the device needs an explicit stage_halves bound")
         Lmax = min(k_store.max_tokens, v_store.max_tokens)
-        # a caller's workspace may be the smallest one (the window in one record); the default one has room for all
-        _, nbytes = plan(n_kv, Lmax, W if workspace is None else 0, group, nsplit)
+        # a caller's workspace may be the smallest one (the window in one record)
+        _, nbytes = plan(n_kv, Lmax, WINDOW_ROOM if workspace is None else 0, group, nsplit)
         ws = _take_workspace(workspace, q.device, nbytes)
         r = _lib.native().mfar_decode_attention_fp16_dyn(
             q.data_ptr(), q.stride(0), n_kv, group,
@@ -239,7 +244,7 @@ def decode_attention(q: torch.Tensor, k_store: SparseStore, v_store: SparseStore
         if _debug_check():
             check_device_status(q.device)
         return out
-    _, nbytes = plan(n_kv, L, W if workspace is None else 0, group, nsplit)
+    _, nbytes = plan(n_kv, L, WINDOW_ROOM if workspace is None else 0, group, nsplit)
     ws = _take_workspace(workspace, q.device, nbytes)
     r = _lib.native().mfar_decode_attention_fp16(
         q.data_ptr(), q.stride(0), n_kv, group,

@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 from .compression import D, _stream
-from .ops import _debug_check, _dev_status, _take_workspace, _workspace, check_device_status, plan
+from .ops import WINDOW_ROOM, _debug_check, _dev_status, _take_workspace, _workspace, check_device_status, plan
 
 
 def _check(bmp, NZ_quant, tile_offsets, scales, zeros, B):
@@ -77,6 +77,11 @@ def mustafar_key_formulation_quant_meta(bmp, NZ_quant, tile_offsets, tile_counts
                                           Batch_Size, num_key_value_groups, bit, capacity, dequant_mode)
 
 
+def _records_bytes(n_kv, n_tokens, group, window=WINDOW_ROOM):
+    """Workspace with a record per 64-token block of the cache and of the window."""
+    return 65536 + n_kv * (max(1, n_tokens // 64) + (window + 63) // 64) * group * 132 * 4
+
+
 def _value(bmp, NZ_quant, tile_offsets, scales, zeros, P, probs_stride, M_Global, K_Global, Batch_Size, groups, bit,
            capacity, out, out_stride, split_k):
     _check(bmp, NZ_quant, tile_offsets, scales, zeros, P)
@@ -84,8 +89,8 @@ def _value(bmp, NZ_quant, tile_offsets, scales, zeros, P, probs_stride, M_Global
         raise RuntimeError("unsupported shape: head_dim 128, K_Global % 64 == 0, bit * capacity == 32")
     n_kv = Batch_Size // groups
     tiles = M_Global * K_Global // 64
-    _, nbytes = plan(n_kv, K_Global, 0, groups)
-    ws = _workspace(P.device, max(nbytes, 65536 + n_kv * max(1, K_Global // 64) * groups * 132 * 4))
+    _, nbytes = plan(n_kv, K_Global, WINDOW_ROOM, groups)
+    ws = _workspace(P.device, max(nbytes, _records_bytes(n_kv, K_Global, groups)))
     st = _dev_status(P.device)
     r = _lib.native().mfar_value_output_rows_quant(
         P.data_ptr(), probs_stride, n_kv, groups, bmp.data_ptr(), tiles, tile_offsets.data_ptr(), scales.data_ptr(),
@@ -153,9 +158,7 @@ def decode_attention_quant(q, kq: dict, vq: dict, n_tokens: int, k_window, v_win
         softmax_scale = 1.0 / math.sqrt(D)
     if out is None:
         out = torch.empty((n_kv * group, D), dtype=torch.float16, device=q.device)
-    # (the default workspace has room for all the records a window may be split into)
-    records = max(1, n_tokens // 64) + (16 if workspace is None else 1)
-    ws = _take_workspace(workspace, q.device, 65536 + n_kv * records * group * 132 * 4)
+    ws = _take_workspace(workspace, q.device, _records_bytes(n_kv, n_tokens, group, WINDOW_ROOM if workspace is None else 1))
     for t, name in ((n_tokens_dev, "n_tokens_dev"), (window_len, "window_len")):
         if t is not None and (not t.is_cuda or t.dtype != torch.int32 or t.numel() != 1):
             raise RuntimeError(f"{name} must be a CUDA int32 tensor with one element")
