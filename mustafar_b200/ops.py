@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes as C
 import functools
 import math
+import operator
 import os
 
 import torch
@@ -88,10 +89,12 @@ def _take_workspace(workspace, device, nbytes: int) -> torch.Tensor:
 
 def plan(n_kv_heads: int, n_tokens: int, window: int, group: int, nsplit: int = 0):
     """(splits, workspace bytes) of a decode call on the current device."""
+    # remembered by value: a 0-d tensor is read now, and a float equal to a remembered size is refused like any other
+    sizes = map(operator.index, (n_kv_heads, n_tokens, window, group, nsplit))
     # without a CUDA context the library plans for a default device, which is not to be remembered
     if not torch.cuda.is_initialized():
-        return _plan.__wrapped__(-1, n_kv_heads, n_tokens, window, group, nsplit)
-    return _plan(torch._C._cuda_getDevice(), n_kv_heads, n_tokens, window, group, nsplit)
+        return _plan.__wrapped__(-1, *sizes)
+    return _plan(torch._C._cuda_getDevice(), *sizes)
 
 
 @functools.lru_cache(maxsize=256)
