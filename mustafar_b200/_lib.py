@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libmustafar_b200.so")
@@ -99,14 +100,16 @@ _native = None
 
 def native():
     """The entry points of the decode step through the CPython binding (csrc/native.cpp): the same functions as
-    ``lib()``'s, at a tenth of the call overhead."""
+    ``lib()``'s, at a tenth of the call overhead.  Where the binding was not built for this interpreter it IS ``lib()``."""
     global _native
     if _native is None:
-        lib()
+        handle = lib()
         try:
             from . import _native as module
         except ImportError as e:
-            raise RuntimeError(f"mustafar_b200/_native.so: {e}; build it with `python -m mustafar_b200.build`") from e
+            warnings.warn(f"mustafar_b200 calls its library through ctypes ({e}); `python -m mustafar_b200.build` builds the "
+                          "binding for this interpreter", RuntimeWarning, stacklevel=2)
+            module = handle
         _native = module
     return _native
 

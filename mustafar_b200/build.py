@@ -1,5 +1,5 @@
-"""Builds libmustafar_b200.so (all CUDA sources of csrc/, sm_100a only) and _native.so (the CPython binding of its
-hot entry points) in-tree with nvcc.
+"""Builds libmustafar_b200.so (all CUDA sources of csrc/, sm_100a only) and, where the interpreter's C headers are
+installed, _native.<ABI tag>.so (the CPython binding of its hot entry points) in-tree with nvcc.
 
     python -m mustafar_b200.build [--force] [--verbose]
 
@@ -21,7 +21,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libmustafar_b200.so")
-NATIVE = os.path.join(HERE, "_native.so")
+# the tag keeps a tree built for one interpreter from loading its binding into another
+NATIVE = os.path.join(HERE, "_native" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]
 
@@ -39,6 +40,24 @@ def _newest_header() -> float:
         if f.endswith((".cuh", ".h")):
             t = max(t, os.path.getmtime(os.path.join(CSRC, f)))
     return t
+
+
+def build_native(nvcc: str, hdr_t: float, force: bool = False) -> str | None:
+    """The binding is a shortcut, not a requirement: without Python.h it is left out and the package calls the same
+    functions through ctypes."""
+    include = sysconfig.get_path("include")
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write(f"no Python.h in {include}: the CPython binding is left out\n")
+        return None
+    src = os.path.join(CSRC, "native.cpp")
+    if force or not os.path.exists(NATIVE) or os.path.getmtime(NATIVE) < max(os.path.getmtime(src), hdr_t):
+        cmd = [nvcc, "-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-cudart", "none", "-o", NATIVE, src,
+               "-I", include, "-L", HERE, "-l:" + os.path.basename(LIB), "-Xlinker", "-rpath=$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("the CPython binding failed to build")
+    return NATIVE
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -75,14 +94,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
-    src = os.path.join(CSRC, "native.cpp")
-    if force or not os.path.exists(NATIVE) or os.path.getmtime(NATIVE) < max(os.path.getmtime(src), hdr_t):
-        cmd = [nvcc, "-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-cudart", "none", "-o", NATIVE, src,
-               "-I", sysconfig.get_path("include"), "-L", HERE, "-l:" + os.path.basename(LIB), "-Xlinker", "-rpath=$ORIGIN"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-            raise RuntimeError("the CPython binding failed to build")
+    build_native(nvcc, hdr_t, force)
     return LIB
 
 
