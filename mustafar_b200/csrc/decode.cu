@@ -432,8 +432,6 @@ static int decode_attention_fp16_impl(
     p.nblk = n_tokens / 64;
     p.cap = pick_cap(stage_halves);
     p.scale_log2 = softmax_scale * 1.4426950408889634f;
-    // more kv heads than counters: the records are merged by a second launch instead
-    p.counters = n_kv_heads <= kMaxCountedHeads ? static_cast<unsigned*>(workspace) : nullptr;
     p.ws = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + counters_bytes(n_kv_heads));
     p.out = static_cast<__half*>(out);
     p.out_stride = out_stride;
@@ -441,6 +439,7 @@ static int decode_attention_fp16_impl(
     p.nsplit = ns;
     p.bps = ns > 0 ? (p.nblk + ns - 1) / ns : 0;
     split_window(p, n_kv_heads, device_sm_count(), static_cast<long long>((workspace_bytes - counters_bytes(n_kv_heads)) / record));
+    p.counters = merge_counters(workspace, n_kv_heads, p.nrec);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     r = launch_decode_attn(p, group, n_kv_heads, p.nrec, s);
     if (r || p.counters) return r;

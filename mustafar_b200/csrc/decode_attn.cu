@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kAThreads, (QBITS != 0 && G == 8) ? 4 : 5) dec
     // warp w merges heads w, w + 4: its lanes fetch the records' (m, l) in parallel, the weights go through shared
     // memory (the reduction buffer is free again), then every lane sums four channels over the records
     const int nrec = p.nrec;
-    float* wgt = red;   // [G][nrec], nrec <= kMaxSplits + kMaxWindowSplits < 4 * kD
+    float* wgt = red;   // [G][nrec], nrec <= kMaxMergedRecords
     for (int g = warp; g < G; g += kAWarps) {
         const float* base = record_ptr(p, G, h, 0, g);
         const int64_t step = static_cast<int64_t>(G) * kPartialStride;

@@ -173,7 +173,8 @@ constexpr int kPartL = kD + 1;
 enum { MODE_KEY = 1, MODE_VALUE = 2 };
 constexpr int kSlackHalves = 64;  // a decode never reads further than this past a stage's values
 constexpr int kMaxBlocksPerSplit = 256;
-constexpr int kMaxSplits = 480;    // per kv head, whatever a caller asks for
+// splits per kv head, whatever a caller asks for; the fp16 cache takes more where kMaxBlocksPerSplit needs them
+constexpr int kMaxSplits = 480;
 
 struct Sparse {
     const unsigned long long* bmp;
@@ -240,6 +241,12 @@ struct DecodeParams {
 constexpr size_t kCounterBytes = 64 * 1024;
 constexpr int kMaxCountedHeads = static_cast<int>(kCounterBytes / 4);
 inline size_t counters_bytes(int) { return kCounterBytes; }
+// the fused kernel's merge keeps a weight per query head and record in its reduction buffer, 4 * kD floats per query head;
+// with more records (or more kv heads than counters) they are merged by a second launch
+constexpr int kMaxMergedRecords = 4 * kD;
+inline unsigned* merge_counters(void* workspace, int n_kv_heads, int nrec) {
+    return n_kv_heads <= kMaxCountedHeads && nrec <= kMaxMergedRecords ? static_cast<unsigned*>(workspace) : nullptr;
+}
 
 // Checks one 64-token block's packed range before it is copied: block start `blk` and end `nxt` in uint32 units
 // (entries of accum), stage capacity `capb` in bytes, start of the head inside nz and the extent of nz in halves.

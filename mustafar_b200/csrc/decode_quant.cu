@@ -496,7 +496,7 @@ extern "C" int mfar_decode_attention_quant(
     p.L_dev = n_tokens_dev;
     p.cap = 8;
     p.scale_log2 = softmax_scale * 1.4426950408889634f;
-    p.counters = n_kv_heads <= kMaxCountedHeads ? static_cast<unsigned*>(workspace) : nullptr;
+    p.counters = merge_counters(workspace, n_kv_heads, p.nrec);
     p.ws = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + counters_bytes(n_kv_heads));
     p.out = static_cast<__half*>(out);
     p.out_stride = out_stride;
