@@ -279,13 +279,18 @@ __device__ __forceinline__ void zero_score_rows(__half* block, int64_t head_stri
         *reinterpret_cast<uint4*>(block + g * head_stride + r * row_stride + 8 * (i & 7)) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
+
 // The dense window of a kv head is dealt out over p.nwin CTAs of p.wbps 64-token blocks.  A window block reads its K and
-// then its V rows straight from global memory, two exposed trips per block, so a CTA with the 5 blocks of 300 tokens
-// outlasts a whole short split.  While the grid stays under 4 CTAs per SM every block gets its own CTA; beyond that a
-// window CTA takes as many blocks as half a split, which saves prologues and records.  One CTA for the whole
-// window against this: 64 sequences x 32768 tokens, window 128, 1327 -> 1311 us; the attention of a step over 4 x 2048 tokens,
-// window 201 of 384, 4 us less; no shape measured slower.  records: what the workspace has room
-// for (at least nsplit + 1).
+// then its V rows straight from global memory, two exposed trips per block, so a CTA with all blocks outlasts a short split
+// (8 kv heads x 1024 tokens, window 384: 20.8 us with one CTA, 10.1 us with six).  A window CTA takes half of a split's
+// blocks, so that it does not outlast one.  More CTAs also cost: where they push a grid of k <= 5 CTAs per SM beyond k, a
+// few SMs with one CTA too many are what the call waits for (8 x 10240, window 128: 18.8 us with one window CTA, 25.4 us with
+// two).  They are then only as many as fit, provided that none gets more than 4/3 of a split's blocks.
+// Measured over 8 .. 256 kv heads, 512 .. 32768 tokens, windows of 65 .. 384, fp16 with 4 and 8 query heads and 2-bit codes
+// (1530 calls): 6.0 % less time on average than one CTA for the window, more than 3 % slower than that in 25 calls (12 % at
+// worst).  The first form, one block per CTA while the grid stayed under 4 CTAs per SM and no look at k: 4.5 % less time,
+// more than 3 % slower in 106 calls (42 % at worst).
+// records: what the workspace has room for (at least nsplit + 1).
 constexpr int kMaxWindowSplits = 16;
 inline int window_records(int window) {
     const int nwb = (window + 63) / 64;
@@ -295,15 +300,23 @@ inline void split_window(DecodeParams& p, int n_kv_heads, int n_sm, long long re
     const int nwb = (p.W + 63) / 64;
     p.nwin = p.wbps = 0;
     if (nwb > 0) {
-        const bool roomy = static_cast<long long>(n_kv_heads) * (p.nsplit + nwb) <= 4ll * n_sm;
-        int wb = roomy ? 1 : (p.bps / 2 < 1 ? 1 : p.bps / 2);
+        const long long fit = static_cast<long long>(n_sm > 0 ? n_sm : 1);
+        auto per_sm = [&](int nwin) { return (static_cast<long long>(n_kv_heads) * (p.nsplit + nwin) + fit - 1) / fit; };
+        auto ctas = [&](int blocks) { return (nwb + blocks - 1) / blocks; };
+        int wb = p.bps / 2 < 1 ? 1 : p.bps / 2;
+        const long long k = per_sm(1);
+        if (k <= 5 && per_sm(ctas(wb)) > k) {
+            const long long room = k * fit / n_kv_heads - p.nsplit;   // >= 1: one window CTA fits
+            const int blocks = ctas(static_cast<int>(room < nwb ? room : nwb));
+            if (3 * blocks <= 4 * p.bps) wb = blocks;
+        }
         long long most = records - p.nsplit;
         if (most > kMaxWindowSplits) most = kMaxWindowSplits;
         const int least = static_cast<int>((nwb + most - 1) / most);
         if (wb < least) wb = least;
         if (wb > nwb) wb = nwb;
         p.wbps = wb;
-        p.nwin = (nwb + wb - 1) / wb;
+        p.nwin = ctas(wb);
     }
     p.nrec = p.nsplit + p.nwin;
 }
