@@ -74,7 +74,8 @@ def test_fp16_tiles(G, L):
     ops.check_device_status()
 
 
-@pytest.mark.parametrize("heads,L", [(2, 0), (2, 192), (300, 64)])          # window CTAs of one block, and of several
+# window CTAs of one block; of several only at W = 1100 and in the smallest workspace (test_gpu_window_split.py has the rest)
+@pytest.mark.parametrize("heads,L", [(2, 0), (2, 192), (300, 64)])
 @pytest.mark.parametrize("W", [1, 63, 64, 65, 129, 300, 1100])
 @pytest.mark.parametrize("bits", [16, 2])
 def test_window_split(heads, L, W, bits):

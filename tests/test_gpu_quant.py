@@ -84,9 +84,12 @@ def test_quant_ops_vs_dequantise_then_dense(m, G, Bh, L, s, bits, group):
     want = oracle.key_formulation_ref(kd, q, G)
     padded = torch.nn.functional.pad(q.cuda().view(Bh * G, 1, 128), (0, 0, 0, 7))
     args = (kq["bitmaps"], kq["packed"], kq["tile_offsets"])
+    for shape in ((Bh * G, 8, L), (Bh * G, 8, 128)):      # the results' memory is not zero beforehand
+        torch.full(shape, float("nan"), dtype=torch.float16, device="cuda")
     out = m.oq.mustafar_key_formulation_quant(*args, kq["scales"], kq["zeros"], padded, L, 128, Bh * G, G, bits, cap, 0)
     assert out.shape == (Bh * G, 8, L)
     assert oracle.rel_l2(out[:, 0].cpu(), want) < TOL
+    assert (out[:, 1:].view(torch.int16) == 0).all()
     out2 = m.oq.mustafar_key_formulation_quant_meta(*args, kq["counts"], kq["units"], kq["scales"], kq["zeros"], padded,
                                                     L, 128, Bh * G, G, bits, cap, 1)
     assert torch.equal(out, out2)
@@ -100,6 +103,7 @@ def test_quant_ops_vs_dequantise_then_dense(m, G, Bh, L, s, bits, group):
     o1 = m.oq.mustafar_value_formulation_quant(*vargs, pp, ws, 128, L, Bh * G, G, bits, cap, 0, 4, 2)
     assert o1.shape == (Bh * G, 8, 128)
     assert oracle.rel_l2(o1[:, 0].cpu(), want_v) < TOL
+    assert (o1[:, 1:].view(torch.int16) == 0).all()
     o2 = m.oq.mustafar_value_formulation_quant_decode_n1(*vargs, p.cuda(), ws, 128, L, Bh * G, G, bits, cap, 0, 4)
     assert o2.shape == (Bh * G, 128)
     assert oracle.rel_l2(o2.cpu(), want_v) < TOL

@@ -1,8 +1,8 @@
 """The allocation-free compression entry point (for hosts that may not call cudaMalloc while
 running, e.g. a server that owns all device memory through its own arena) must write exactly what
-the regular entry point writes.  Called straight through the C ABI, twice in a row with different
-inputs, because both calls share one scratch array inside the library and the second must not be
-disturbed by what the first left there."""
+the regular entry point writes.  Called straight through the C ABI, several times in a row with different
+inputs, because the calls share one scratch array inside the library and the next must not be
+disturbed by what the ones before left there."""
 import pytest
 import torch
 
@@ -35,7 +35,8 @@ def test_noalloc_entry_matches_regular_entry_twice():
     from mustafar_b200 import _lib
     lib = _lib.lib()
     g = torch.Generator(device="cuda").manual_seed(11)
-    shapes = [((6, 1024, 128), 0, 89), ((3, 448, 128), 1, 64)]     # (shape, kind, prune rank); two calls in a row
+    # (shape, kind, prune rank), in a row; 448 tokens run as clusters and leave the scratch array alone, the others use it
+    shapes = [((6, 1024, 128), 0, 89), ((3, 448, 128), 1, 64), ((3, 704, 128), 1, 64), ((5, 960, 128), 0, 100)]
     for shape, kind, rank in shapes:
         x = torch.randn(shape, generator=g, device="cuda").half()
         want = _run(lib, x, kind, rank, "regular")
