@@ -333,8 +333,9 @@ extern "C" int mfar_compress_fp16(const void* x, int64_t x_head_stride, int64_t 
     if (static_cast<int64_t>(n_heads) * nblk > 0x7fffffffll) return MFAR_ERR_LIMIT;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // a cluster per head up to the portable cluster size: 256 heads x 256 tokens of K and of V
-    // take 33.3 us against 39.0 us with the look-back (a memset, tickets and polls less)
+    // a cluster per head up to the portable cluster size (a memset, tickets and polls less): 256 heads x 256 tokens of K and
+    // of V take 33.3 us against 39.0 us with the look-back.  Over 1 .. 512 heads x 1 .. 8 blocks, K and V: 0.51 (128 x 3) to
+    // 0.99 (512 x 7) of its time, so the line is the cluster size itself
     const bool cluster = nblk <= kClusterBlocks;
     if (!cluster && !cuda_ok(cudaMemsetAsync(scratch, 0, need, s))) return MFAR_ERR_LAUNCH;
 

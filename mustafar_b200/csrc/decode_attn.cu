@@ -17,8 +17,11 @@
 // The two positions of a register are told apart by the B operand (BForms in decode_common.cuh): up to 4 query heads
 // fill the 8 columns twice, 8 heads take two instructions.  Against registers that pair two TILES this halves the
 // accumulators of up to 4 heads (128 -> 96 registers, 5 CTAs per SM instead of 4) and the score stores: 64 sequences x
-// 32768 tokens, 4 heads per kv head, 1361 -> 1327 us; 7 x 10176 tokens, 8 heads, 110 -> 106 us.  What bounds the kernel
-// now is the shared-memory traffic of the predicated loads (72 % of the data pipe, 61 % of the issue slots).
+// 32768 tokens, 4 heads per kv head, 1361 -> 1327 us; 7 x 10176 tokens, 8 heads, 110 -> 106 us.  Over 360
+// shapes each (8 .. 512 kv heads x 256 .. 32768 tokens, window dealt out) 2, 4 and 8 heads take 10, 10 and 6 % less time than
+// that form, one head 7 % less, but 3 .. 8 % more at 16 .. 56 kv heads x 4096 tokens and up (4 CTAs per SM with 128 registers
+// there: 4 % more over all shapes).  What the kernel waits for now is the shared-memory traffic of the
+// predicated loads: 71 % of the data pipe, 62 % of the issue slots, neither saturated.
 //
 // The same kernel serves the quantised cache (QBITS = 2 or 4): there a tile's code words, bitmap, scale and zero-point
 // are staged by the threads themselves (4-byte cp.async, one tile of each tensor per thread, one block ahead); a lane
@@ -28,7 +31,8 @@
 // reference's arithmetic (kernel_quant/csrc/SpMM_Kernel_Quant.cuh:235-240) -, 4-bit codes by an exact fp16 subtraction
 // and one rounded product, which gives the same bits (zero-points outside +-1024 go through fp32).  Against one
 // predicated step per position: 32 x 16384 tokens of 2-bit codes 583 -> 450 us, 8 x 4096 of 4-bit codes with a scale per
-// 32 nonzeros, half of the values kept, 82.7 -> 69.6 us.  Bound by the integer pipe and issue (both about 60 %).
+// 32 nonzeros, half of the values kept, 82.7 -> 69.6 us.  The integer pipe, issue and the shared-memory pipe are each used
+// to about 60 %.
 #include "decode_plain.cuh"
 
 namespace mfar {

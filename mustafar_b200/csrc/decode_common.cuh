@@ -322,15 +322,20 @@ inline void split_window(DecodeParams& p, int n_kv_heads, int n_sm, long long re
 }
 
 // Split count of the 64-token-block decode kernels.  The grid is n_kv_heads * ns CTAs of bps = ceil(nblk / ns) blocks.
-// The cost of a candidate follows a model fitted to a measured sweep of ns over batch 1..64 and
-// 4k..32k tokens on a B200 (all times in units of one block on an otherwise idle SM, ~2 us):
+// The cost of a candidate follows a model fitted to a sweep of ns over batch 1..64 and 4k..32k tokens with the kernel that
+// had 4 CTAs per SM and one window CTA (all times in units of one block on an otherwise idle SM, ~2 us):
 //   * a CTA costs w = bps + 1.1 (prologue, partial record);
 //   * x = CTAs / SMs is the load per SM; an SM's throughput with o = min(x, 4) resident CTAs is
 //     rate(o) = 1 / 2 / 2.76 / 2.13 at o = 1 / 2 / 3 / 4, linear in between (the dip at 4 is the fit's
 //     way of saying that a grid which fits in one not-quite-full wave beats one that needs two);
 //   * the last, partly filled wave costs another 0.8 w once the SMs hold more than one CTA;
 //   * merging the records adds 0.035 per record.
-// The pick stays within 2 % of the best swept ns on every measured shape.
+// The kernels have changed since (5 CTAs per SM for most, window CTAs, cheaper codes).  Measured with them over 150 shapes
+// (8 .. 512 kv heads x 1024 .. 32768 tokens, window 128, 1, 4 and 8 query heads, fp16 and 2-bit): the pick costs 2.3 % more
+// than the best swept ns on average, more than 2 % in 38 of them, at worst 12 % for fp16 (256 kv heads x 1024 tokens, 1 query
+// head: 2 splits, 4 are better) and 22 % for 2-bit codes (8 x 1024: 16 splits of the model, of which the quantised call uses
+// half).  A refit to 5 CTAs per SM gave 2.4 % instead of 4.3 % over 136 shapes but made 7 x 10176 tokens with 8 query heads
+// 106 -> 114 us and 8 x 4096 of 4-bit codes 70 -> 79 us: one model does not fit all variants.
 inline int model_split_count(int n_kv_heads, int nblk, int min_ns, int max_ns, int n_sm) {
     if (max_ns > nblk) max_ns = nblk;
     if (min_ns < 1) min_ns = 1;
